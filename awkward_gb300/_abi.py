@@ -90,6 +90,17 @@ def ext_cfunc(name):
     return f
 
 
+def read_words(stream, *addresses):
+    """The int64 device words at `addresses`, read with one wait for `stream`
+    (a raw cudaStream_t)."""
+    n = len(addresses)
+    src, dst = (ctypes.c_void_p * n)(*addresses), (ctypes.c_int64 * n)()
+    rc = ext_cfunc("awkward_gb300_read_words")(ctypes.addressof(dst), ctypes.addressof(src), n, stream)
+    if rc != 0:
+        raise RuntimeError(f"awkward_gb300_read_words: cudaError {rc}")
+    return list(dst)
+
+
 def exported_symbols():
     """Names declared in include/awkward_gb300.h that the loaded library exports."""
     lib = load_library()

@@ -74,6 +74,11 @@ kernel-specification.yml):
   jagged_index_select: array[index] with a jagged int64 index in one pass
     -- jagged_apply with the content gathered at each carry (itemsize 1, 2,
     4 or 8; tocarry NULL to skip), errors as jagged_apply's;
+  jagged_range_select: array[..., start:stop:step] on one level of lists in
+    one pass -- next_range with the content gathered at each carry (itemsize
+    1, 2, 4 or 8; absent bounds INT64_MAX); tooffsets[nlists] is the number
+    selected, of which the first tolen are written; an element outside
+    [0, contentlen) sets err_code to 0 ("index out of range");
   take: out[i] = content[carry[i]] for itemsize 1, 2, 4 or 8 bytes
     (NumpyArray._carry); a carry outside [0, contentlen) sets err_code to
     invocation_index*256 + 0 ("index out of range")."""
@@ -93,6 +98,11 @@ EXTENSIONS["awkward_gb300_jagged_index_select"] = (
      ("const int64_t*", "offsets"), ("const void*", "content"), ("int64_t", "itemsize"),
      ("int64_t", "contentlen"), ("int64_t", "nlists"), ("uint64_t*", "err_code"),
      ("void*", "stream")], "jagged")
+EXTENSIONS["awkward_gb300_jagged_range_select"] = (
+    [("int64_t*", "tooffsets"), ("void*", "tocontent"), ("int64_t", "tolen"),
+     ("const int64_t*", "offsets"), ("const void*", "content"), ("int64_t", "itemsize"),
+     ("int64_t", "contentlen"), ("int64_t", "nlists"), ("int64_t", "start"), ("int64_t", "stop"),
+     ("int64_t", "step"), ("uint64_t*", "err_code"), ("void*", "stream")], "jagged")
 EXTENSIONS["awkward_gb300_take"] = (
     [("void*", "out"), ("const void*", "content"), ("int64_t", "itemsize"),
      ("const int64_t*", "carry"), ("int64_t", "n"), ("int64_t", "contentlen"),
@@ -156,6 +166,13 @@ EXTENSIONS["awkward_gb300_fused_reduce_float64"] = (
      ("int64_t", "reduce"), ("uint64_t", "invocation_index"), ("uint64_t*", "err_code"),
      ("void*", "stream")], "fused")
 
+_READ_COMMENT = """a few device words to the host (no counterpart in awkward): dst[i] =
+*src[i], at most 16 of them, with one wait for the stream."""
+
+EXTENSIONS["awkward_gb300_read_words"] = (
+    [("int64_t*", "dst"), ("const int64_t* const*", "src"), ("int64_t", "n"),
+     ("void*", "stream")], "read")
+
 _SELFTEST_COMMENT = """self-test of the failure report (no counterpart in awkward): one warp
 runs the decoupled look-back of the scan kernels on tile 1 of a fresh
 scan whose tile 0 never publishes, with a spin limit of `spin_limit`
@@ -172,14 +189,14 @@ EXTENSIONS["awkward_gb300_selftest_lookback_timeout"] = (
 GROUP_COMMENTS = {"noalloc": _NOALLOC_COMMENT, "autograd": _AUTOGRAD_COMMENT,
                   "jagged": _JAGGED_COMMENT, "batch": _BATCH_COMMENT,
                   "pipeline": _PIPELINE_COMMENT, "fused": _FUSED_COMMENT,
-                  "selftest": _SELFTEST_COMMENT}
+                  "read": _READ_COMMENT, "selftest": _SELFTEST_COMMENT}
 GROUP_DEFINES = {"noalloc": ["#define AWKWARD_GB300_NOALLOC_MAX_LISTS 67108864LL"]}
 
 
 def header_lines():
     """Declarations of the extension entry points, grouped, for the C header."""
     out = []
-    for group in ("noalloc", "jagged", "autograd", "batch", "pipeline", "fused", "selftest"):
+    for group in ("noalloc", "jagged", "autograd", "batch", "pipeline", "fused", "read", "selftest"):
         out.append("")
         text = GROUP_COMMENTS[group].splitlines()
         out.append(f"/* ---- {text[0]}")

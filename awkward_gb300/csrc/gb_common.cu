@@ -52,6 +52,20 @@ cudaError_t scratch_free(void* ptr, cudaStream_t stream) {
   return cudaFreeAsync(ptr, stream);
 }
 
+cudaError_t readback(Readback** out) {
+  static thread_local Readback cache[kMaxDevices];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+  Readback& r = cache[dev];
+  if (!r.words)
+    e = cudaHostAlloc((void**)&r.words, sizeof(unsigned long long) * Readback::kWords, cudaHostAllocDefault);
+  if (e == cudaSuccess && !r.done) e = cudaEventCreateWithFlags(&r.done, cudaEventDisableTiming);
+  *out = &r;
+  return e;
+}
+
 int device_sm_count() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 1;
@@ -77,6 +91,22 @@ cudaError_t scan_tiles_alloc(ScanTiles* st, void** base, long long ntiles, cudaS
 }
 
 }  // namespace gb
+
+// dst[i] (host) = *src[i] (int64 device words), n <= 16, once `stream` has got
+// there: one wait for all of them.
+GB_EXPORT int awkward_gb300_read_words(int64_t* dst, const int64_t* const* src, int64_t n,
+                                       void* stream) {
+  if (n < 0 || n > gb::Readback::kWords) return (int)cudaErrorInvalidValue;
+  cudaStream_t s = (cudaStream_t)stream;
+  gb::Readback* r = nullptr;
+  cudaError_t e = gb::readback(&r);
+  for (int64_t i = 0; i < n && e == cudaSuccess; i++)
+    e = cudaMemcpyAsync(r->words + i, src[i], sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+  cudaError_t w = cudaStreamSynchronize(s);  // also before the buffer is used again
+  if (e == cudaSuccess) e = w;
+  for (int64_t i = 0; i < n && e == cudaSuccess; i++) dst[i] = (int64_t)r->words[i];
+  return (int)e;
+}
 
 // Library identification for the host-side loader.
 GB_EXPORT const char* awkward_gb300_version() { return "awkward_gb300 0.1 (sm_103a)"; }

@@ -37,6 +37,16 @@ __device__ __forceinline__ void raise_error(uint64_t* err, uint64_t inv, int cod
 // Stream-ordered allocation from a per-device pool owned by the library.
 cudaError_t scratch_alloc(void** ptr, size_t bytes, cudaStream_t stream);
 cudaError_t scratch_free(void* ptr, cudaStream_t stream);
+// A few device words on their way to the host: a pinned buffer, so that the
+// copies are queued, and an event to wait for them (kernels queued behind it
+// run meanwhile).  One per thread and device; whoever takes it has done with
+// it before it returns.
+struct Readback {
+  static constexpr int kWords = 16;
+  unsigned long long* words = nullptr;
+  cudaEvent_t done = nullptr;
+};
+cudaError_t readback(Readback** out);
 // SM count and the persistent-grid width of the current device (cached).
 int device_sm_count();
 

@@ -46,18 +46,26 @@ __global__ void __launch_bounds__(kTileBlock)
                         long long contentlen, ScanTiles st, uint64_t inv, uint64_t* err,
                         void* __restrict__ tocontent = nullptr,
                         const void* __restrict__ content = nullptr) {
+  // a list's first index less its first slot, its first element and its length
+  struct Lists {
+    long long slice, start, count;
+  };
   __shared__ TileSmem sm;
-  __shared__ long long s_slice[kTileLists];
-  __shared__ long long s_start[kTileLists];
-  __shared__ long long s_count[kTileLists];
+  __shared__ union {
+    struct {
+      long long slice[kTileLists], start[kTileLists], count[kTileLists];
+    } all;              // by list
+    SlotMap<Lists> map;  // by non-empty index list
+  } u;
   const long long tile = tile_claim(sm, st);
+  Lists mine[kTileLPT];
   const long long l0 = tile * kTileLists;
   long long cnt[kTileLPT];
 #pragma unroll
   for (int r = 0; r < kTileLPT; r++) {
-    const int li = threadIdx.x * kTileLPT + r;
-    const long long i = l0 + li;
+    const long long i = l0 + threadIdx.x * kTileLPT + r;
     long long c = 0;
+    mine[r] = {0, 0, 0};
     if (i < n) {
       const long long ss = slicestarts[i], se = slicestops[i];
       const long long start = (long long)fromstarts[i], stop = (long long)fromstops[i];
@@ -69,9 +77,7 @@ __global__ void __launch_bounds__(kTileBlock)
         else if (start != stop && stop > contentlen) { raise_error(err, inv, 3); ok = false; }
         if (ok) c = se - ss;
       }
-      s_slice[li] = ss;
-      s_start[li] = start;
-      s_count[li] = stop - start;
+      mine[r] = {ss, start, stop - start};
     }
     cnt[r] = c;
   }
@@ -83,27 +89,77 @@ __global__ void __launch_bounds__(kTileBlock)
     if (i == n) tooffsets[n] = prefix + total;  // only the tile holding list n-1 ... n
   }
   if (l0 + kTileLists == n && threadIdx.x == 0) tooffsets[n] = prefix + total;
-  tile_for_each_slot(sm, total, [&](long long q, int r) {
-    const long long j = s_slice[r] + (q - sm.loc[r]);
-    long long idx = sliceindex[j];
-    const long long count = s_count[r];
+  // slot q takes index j of a list: false, with the error raised, when it is
+  // out of range
+  auto resolve = [&](long long idx, long long start, long long count, long long* at) {
     if (idx < -count || idx >= count) {
       raise_error(err, inv, 4);
-      return;
+      return false;
     }
-    if (idx < 0) idx += count;
-    const long long at = s_start[r] + idx;
-    if constexpr (std::is_void<W>::value) {
-      tocarry[prefix + q] = at;
-    } else {
-      if (at < 0 || at >= contentlen) {  // a start below zero; the CPU kernel does not check it
+    *at = start + (idx < 0 ? idx + count : idx);
+    if constexpr (!std::is_void<W>::value) {
+      if (*at < 0 || *at >= contentlen) {  // a start below zero; the CPU kernel does not check it
         raise_error(err, inv, 3);
-        return;
+        return false;
       }
-      static_cast<W*>(tocontent)[prefix + q] = __ldg(static_cast<const W*>(content) + at);
-      if (tocarry) tocarry[prefix + q] = at;
     }
+    return true;
+  };
+  if (total > kMapSlots) {
+#pragma unroll
+    for (int r = 0; r < kTileLPT; r++) {
+      const int li = threadIdx.x * kTileLPT + r;
+      u.all.slice[li] = mine[r].slice;
+      u.all.start[li] = mine[r].start;
+      u.all.count[li] = mine[r].count;
+    }
+    __syncthreads();
+    tile_for_each_slot(sm, total, [&](long long q, int r) {
+      long long at;
+      if (!resolve(sliceindex[u.all.slice[r] + (q - sm.loc[r])], u.all.start[r], u.all.count[r], &at)) return;
+      if constexpr (!std::is_void<W>::value)
+        static_cast<W*>(tocontent)[prefix + q] = __ldg(static_cast<const W*>(content) + at);
+      if (std::is_void<W>::value || tocarry) tocarry[prefix + q] = at;
+    });
+    return;
+  }
+  slot_map(u.map, sm, (int)total, cnt, [&](int li) {
+    Lists v = mine[li % kTileLPT];
+    v.slice -= sm.loc[li];
+    return v;
   });
+  // four slots per thread and step: their index loads, then their content
+  // loads, are in flight together
+  constexpr int kUnroll = 4;
+  for (int q0 = threadIdx.x; q0 < (int)total; q0 += kUnroll * kTileBlock) {
+    long long idx[kUnroll], at[kUnroll];
+    Lists l[kUnroll];
+    bool ok[kUnroll];
+#pragma unroll
+    for (int k = 0; k < kUnroll; k++) {
+      const int q = q0 + k * kTileBlock;
+      ok[k] = q < (int)total;
+      if (ok[k]) {
+        l[k] = slot_of(u.map, q);
+        idx[k] = __ldg(sliceindex + (l[k].slice + q));
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kUnroll; k++)
+      if (ok[k]) ok[k] = resolve(idx[k], l[k].start, l[k].count, &at[k]);
+    if constexpr (!std::is_void<W>::value) {
+      W v[kUnroll];
+#pragma unroll
+      for (int k = 0; k < kUnroll; k++)
+        if (ok[k]) v[k] = __ldg(static_cast<const W*>(content) + at[k]);
+#pragma unroll
+      for (int k = 0; k < kUnroll; k++)
+        if (ok[k]) static_cast<W*>(tocontent)[prefix + q0 + k * kTileBlock] = v[k];
+    }
+#pragma unroll
+    for (int k = 0; k < kUnroll; k++)
+      if (ok[k] && (std::is_void<W>::value || tocarry)) tocarry[prefix + q0 + k * kTileBlock] = at[k];
+  }
 }
 
 // ------------------------------------------------------------------ carrylen

@@ -146,6 +146,68 @@ __device__ __forceinline__ void tile_for_each_slot(const TileSmem& sm, long long
   }
 }
 
+// Slots to lists of a tile with at most kMapSlots output slots: a bitmap of the
+// slots where a list begins, the begins before each of its words, and per begin
+// (the non-empty lists, in order) what the fill needs of its list.  A slot's
+// list is then one broadcast word, one popcount and one look-up, whatever the
+// lengths are, and a thread can have several slots in flight, where
+// warp_step_lists takes one step after another: the carry of [..., 1:] over 4M
+// lists of mean 6 went from 104 to 96 us.
+constexpr int kMapSlots = 16384;
+template <class V>
+struct SlotMap {
+  unsigned bits[kMapSlots / 32];
+  unsigned short before[kMapSlots / 32];
+  V of[kTileLists];  // by begin
+  unsigned scan[kTileBlock / 32 + 1];
+};
+
+// Build the map of a scanned tile (all threads; total <= kMapSlots): value(r)
+// is stored for list r of the tile with a count above 0.
+template <class V, class Value>
+__device__ __forceinline__ void slot_map(SlotMap<V>& m, const TileSmem& sm, int total,
+                                         const long long (&cnt)[kTileLPT], Value value) {
+  constexpr int kPer = kMapSlots / 32 / kTileBlock;
+  const int words = (total + 31) >> 5;
+  for (int w = threadIdx.x; w < words; w += kTileBlock) m.bits[w] = 0u;
+  unsigned mine = 0;
+#pragma unroll
+  for (int r = 0; r < kTileLPT; r++) mine += cnt[r] > 0;
+  unsigned all;
+  auto add = [](unsigned a, unsigned b) { return a + b; };
+  unsigned rank = block_exclusive_scan<kTileBlock>(mine, add, 0u, m.scan, &all);
+#pragma unroll
+  for (int r = 0; r < kTileLPT; r++) {
+    if (cnt[r] <= 0) continue;
+    const int li = threadIdx.x * kTileLPT + r, at = (int)sm.loc[li];
+    atomicOr(m.bits + (at >> 5), 1u << (at & 31));
+    m.of[rank++] = value(li);
+  }
+  __syncthreads();
+  unsigned n[kPer], sum = 0;
+#pragma unroll
+  for (int i = 0; i < kPer; i++) {
+    const int w = threadIdx.x * kPer + i;
+    n[i] = w < words ? __popc(m.bits[w]) : 0u;
+    sum += n[i];
+  }
+  unsigned run = block_exclusive_scan<kTileBlock>(sum, add, 0u, m.scan, &all);
+#pragma unroll
+  for (int i = 0; i < kPer; i++) {
+    const int w = threadIdx.x * kPer + i;
+    if (w < words) m.before[w] = (unsigned short)run;
+    run += n[i];
+  }
+  __syncthreads();
+}
+
+// The map's entry of slot q.
+template <class V>
+__device__ __forceinline__ V slot_of(const SlotMap<V>& m, int q) {
+  const unsigned le = 0xffffffffu >> (31 - (q & 31));
+  return m.of[m.before[q >> 5] + __popc(m.bits[q >> 5] & le) - 1];
+}
+
 // Stage the tile of lists [l0, l0 + kTileLists) (those below n): sm.loc holds
 // the local exclusive offsets of their (non-negative) counts; returns the
 // tile's total count.  All threads call it.

@@ -7,6 +7,8 @@
 // Each list's slice is clipped against the list's length exactly as
 // kernel-utils.cpp:7-39 (awkward_regularize_rangeslice) does; the number of
 // kept positions is then computed in closed form instead of by stepping.
+#include <type_traits>
+
 #include "list_tile.cuh"
 
 using namespace gb;
@@ -76,13 +78,26 @@ __device__ __forceinline__ long long range_count(long long length, long long sta
   return span / astep + 1;
 }
 
-template <class C>
+// Four slots per thread and step: their loads are issued together.
+constexpr int kFillUnroll = 4;
+
+// With W other than void the fill gathers the content at each carry into
+// tocontent (its first tolen places) instead of writing the carry.
+//
+// 4M lists of mean 6 (float64), [..., 1:]: 111 us for the selection in one
+// kernel, against 22 + 96 + 69 us for the count, the carry and its gather.
+// Bound by the tile's chain of barriers (loads, scan, look-back, map) and its
+// instructions; DRAM traffic is the offsets and the content once.
+template <class C, class W = void>
 __global__ void __launch_bounds__(kTileBlock)
     next_range_kernel(C* __restrict__ tooffsets, int64_t* __restrict__ tocarry,
                       const C* __restrict__ fromstarts, const C* __restrict__ fromstops,
                       long long n, long long start, long long stop, long long step, ScanTiles st,
-                      uint64_t inv, uint64_t* err) {
+                      uint64_t inv, uint64_t* err, void* __restrict__ tocontent = nullptr,
+                      const void* __restrict__ content = nullptr, long long contentlen = 0,
+                      long long tolen = 0) {
   __shared__ TileSmem sm;
+  __shared__ SlotMap<long long> map;         // fromstarts[i] + regular start - first slot * step
   __shared__ long long s_first[kTileLists];  // fromstarts[i] + regular start
   const long long tile = tile_claim(sm, st);
   const long long l0 = tile * kTileLists;
@@ -108,9 +123,48 @@ __global__ void __launch_bounds__(kTileBlock)
     if (i < n) tooffsets[i + 1] = (C)(prefix + sm.loc[li + 1]);
   }
   if (tile == 0 && threadIdx.x == 0) tooffsets[0] = 0;
-  tile_for_each_slot(sm, total, [&](long long q, int r) {
-    tocarry[prefix + q] = s_first[r] + (q - sm.loc[r]) * step;
-  });
+  auto put = [&](long long q, long long at) {
+    if constexpr (std::is_void<W>::value) {
+      tocarry[prefix + q] = at;
+    } else {
+      if (at < 0 || at >= contentlen) raise_error(err, inv, 0);
+      else if (prefix + q < tolen)
+        static_cast<W*>(tocontent)[prefix + q] = __ldg(static_cast<const W*>(content) + at);
+    }
+  };
+  if (total > kMapSlots) {
+    tile_for_each_slot(sm, total, [&](long long q, int r) { put(q, s_first[r] + (q - sm.loc[r]) * step); });
+    return;
+  }
+  slot_map(map, sm, (int)total, cnt, [&](int r) { return s_first[r] - sm.loc[r] * step; });
+  for (int q0 = threadIdx.x; q0 < (int)total; q0 += kFillUnroll * kTileBlock) {
+    long long at[kFillUnroll];
+#pragma unroll
+    for (int u = 0; u < kFillUnroll; u++) {
+      const int q = q0 + u * kTileBlock;
+      at[u] = q < (int)total ? slot_of(map, q) + q * step : -1;
+    }
+    if constexpr (std::is_void<W>::value) {
+#pragma unroll
+      for (int u = 0; u < kFillUnroll; u++) {
+        const int q = q0 + u * kTileBlock;
+        if (q < (int)total) tocarry[prefix + q] = at[u];
+      }
+    } else {
+      W v[kFillUnroll];
+#pragma unroll
+      for (int u = 0; u < kFillUnroll; u++) {
+        const bool in = at[u] >= 0 && at[u] < contentlen;
+        v[u] = in ? __ldg(static_cast<const W*>(content) + at[u]) : W(0);
+        if (!in && q0 + u * kTileBlock < (int)total) raise_error(err, inv, 0);
+      }
+#pragma unroll
+      for (int u = 0; u < kFillUnroll; u++) {
+        const int q = q0 + u * kTileBlock;
+        if (q < (int)total && prefix + q < tolen) static_cast<W*>(tocontent)[prefix + q] = v[u];
+      }
+    }
+  }
 }
 
 template <class C>
@@ -197,4 +251,40 @@ GB_EXPORT int awkward_RegularArray_getitem_next_range_64(int64_t* tocarry, int64
   regular_next_range_kernel<<<map_grid(total), kMapBlock, 0, (cudaStream_t)stream>>>(
       tocarry, regular_start, step, length, size, nextsize);
   return (int)cudaGetLastError();
+}
+
+// array[..., start:stop:step] on lists content[offsets[i] .. offsets[i+1]) in
+// one pass: the next-range kernel with the content gathered at each carry,
+// which is neither written nor read back.  A list that reaches past the
+// content raises code 0 ("index out of range"), as the carry's take does.
+// tooffsets[nlists] is the number of selected elements; only the first tolen
+// are written (at most the elements of the lists' span unless offsets decrease).
+GB_EXPORT int awkward_gb300_jagged_range_select(int64_t* tooffsets, void* tocontent, int64_t tolen,
+                                                const int64_t* offsets, const void* content,
+                                                int64_t itemsize, int64_t contentlen,
+                                                int64_t nlists, int64_t start, int64_t stop,
+                                                int64_t step, uint64_t* err_code, void* stream) {
+  cudaStream_t s = (cudaStream_t)stream;
+  if (itemsize != 1 && itemsize != 2 && itemsize != 4 && itemsize != 8)
+    return (int)cudaErrorInvalidValue;
+  if (nlists <= 0) return (int)cudaMemsetAsync(tooffsets, 0, sizeof(int64_t), s);
+  const long long nt = tile_count(nlists);
+  ScanTiles st;
+  void* base = nullptr;
+  cudaError_t e = scan_tiles_alloc(&st, &base, nt, s);
+  if (e != cudaSuccess) return (int)e;
+#define GB_RANGE_SELECT(W)                                                                   \
+  next_range_kernel<int64_t, W><<<(unsigned)nt, kTileBlock, 0, s>>>(                         \
+      tooffsets, nullptr, offsets, offsets + 1, nlists, start, stop, step, st, 0, err_code,  \
+      tocontent, content, contentlen, tolen)
+  switch (itemsize) {
+    case 1: GB_RANGE_SELECT(uint8_t); break;
+    case 2: GB_RANGE_SELECT(uint16_t); break;
+    case 4: GB_RANGE_SELECT(uint32_t); break;
+    default: GB_RANGE_SELECT(uint64_t);
+  }
+#undef GB_RANGE_SELECT
+  e = cudaGetLastError();
+  cudaError_t f = scratch_free(base, s);
+  return (int)(e != cudaSuccess ? e : f);
 }

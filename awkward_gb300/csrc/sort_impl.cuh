@@ -53,6 +53,7 @@ static_assert(kSortBlock * kMidItems >= kMidWindow - 1 + kMidMax, "a tile fits i
 // the count before it).
 enum { kCntMidTotal = 0, kCntLong = 1, kCntLongTotal = 2, kCntLongMax = 3, kCntLimit = 4,
        kCntWords = 8 };
+static_assert(kCntWords <= Readback::kWords, "the counters are read back in one piece");
 
 // ------------------------------------------------------------ order keys
 template <class T>
@@ -1068,27 +1069,6 @@ __global__ void __launch_bounds__(kSortBlock)
   }
 }
 
-// Where the counters are read back to: pinned, so that the copy is queued
-// between two kernels and only the event is waited for.  One per thread and
-// device; a call has done with it when it returns.
-struct CountReadback {
-  unsigned long long* words = nullptr;
-  cudaEvent_t done = nullptr;
-};
-inline cudaError_t count_readback(CountReadback** out) {
-  constexpr int kDevices = 64;
-  static thread_local CountReadback cache[kDevices];
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= kDevices) return cudaErrorInvalidDevice;
-  CountReadback& c = cache[dev];
-  if (!c.words) e = cudaHostAlloc((void**)&c.words, sizeof(unsigned long long) * kCntWords, cudaHostAllocDefault);
-  if (e == cudaSuccess && !c.done) e = cudaEventCreateWithFlags(&c.done, cudaEventDisableTiming);
-  *out = &c;
-  return e;
-}
-
 template <class T, bool ARG, class P>
 cudaError_t sort_long(void* toptr, const T* x, const SortLists& ls, long long nlong, long long total,
                       long long maxl, bool asc, uint64_t inv, uint64_t* err, cudaStream_t s) {
@@ -1177,9 +1157,9 @@ cudaError_t launch_sort(void* toptr, const T* x, long long length, const U* offs
         toptr, x, length, offsets, nseg, ascending, ls);
     e = cudaGetLastError();
   }
-  CountReadback* rb = nullptr;
+  Readback* rb = nullptr;
   if (e == cudaSuccess && length > kMidMax) {
-    e = count_readback(&rb);
+    e = readback(&rb);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(rb->words, ls.counters, sizeof(long long) * kCntWords, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaEventRecord(rb->done, s);

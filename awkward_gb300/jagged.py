@@ -13,7 +13,8 @@ kernels, for CUDA tensors:
   with the content gathered at each carry), ``mask_select`` the same for
   ``array[mask]``;
 * ``getitem_inner_range``  -- ``array[..., start:stop:step]`` on the innermost
-  list level of a two-level ListOffsetArray:
+  list level of a two-level ListOffsetArray, in one kernel (``range_select``);
+  ``inner_range`` and ``take`` are awkward's own steps:
   ``awkward_ListArray_getitem_next_range_carrylength``, the carry allocation,
   ``awkward_ListArray_getitem_next_range`` and the carry
   (src/awkward/contents/listarray.py:795-862).
@@ -42,9 +43,8 @@ def _err_word(device):
     return torch.full((1,), -1, dtype=torch.int64, device=device)
 
 
-def _raise_if(err, what):
-    word = int(err.item()) & ((1 << 64) - 1)
-    if word != (1 << 64) - 1:
+def _raise_if(word, what):
+    if word != -1:
         raise ValueError(f"index out of range in compiled CUDA code ({what})")
 
 
@@ -58,7 +58,7 @@ def take(content, carry, check=True):
     if rc != 0:
         raise RuntimeError(f"awkward_gb300_take: cudaError {rc}")
     if check:
-        _raise_if(err, "take")
+        _raise_if(int(err.item()), "take")
     return out
 
 
@@ -181,8 +181,47 @@ def inner_range(inner_offsets, start=None, stop=None, step=None):
     return nextoffsets, nextcarry[: int(carrylength.item())]
 
 
+# Up to this many bytes a selection is written into a buffer as long as the
+# content, so that its size need not be counted first.
+_WHOLE_CONTENT = 1 << 30
+
+
+def range_select(inner_offsets, content, start=None, stop=None, step=None):
+    """(nextoffsets, selected content) of [start:stop:step] on every list of one
+    level in one pass (awkward_gb300_jagged_range_select): inner_range and take
+    without writing and re-reading the carry."""
+    n = inner_offsets.numel() - 1
+    bounds = (SLICE_NONE if start is None else start, SLICE_NONE if stop is None else stop,
+              1 if step is None else step)
+    nextoffsets = torch.empty(n + 1, dtype=torch.int64, device=inner_offsets.device)
+    size = content.numel()
+    counted = size * content.element_size() > _WHOLE_CONTENT
+    if counted:
+        be = backend()
+        total = torch.empty(1, dtype=torch.int64, device=inner_offsets.device)
+        be["awkward_ListArray_getitem_next_range_carrylength", np.int64, np.int64, np.int64](
+            total, inner_offsets[:-1], inner_offsets[1:], n, *bounds)
+        be.synchronize()
+        size = int(total.item())
+    while True:
+        out = torch.empty(max(size, 1), dtype=content.dtype, device=content.device)
+        err = _err_word(content.device)
+        rc = _abi.ext_cfunc("awkward_gb300_jagged_range_select")(
+            nextoffsets.data_ptr(), out.data_ptr(), size, inner_offsets.data_ptr(),
+            content.data_ptr(), content.element_size(), content.numel(), n, *bounds,
+            err.data_ptr(), _stream(content))
+        if rc != 0:
+            raise RuntimeError(f"awkward_gb300_jagged_range_select: cudaError {rc}")
+        k, word = _abi.read_words(_stream(content), nextoffsets.data_ptr() + 8 * n, err.data_ptr())
+        _raise_if(word, "take")
+        if k <= size:
+            break
+        size = k  # overlapping lists: more selected than the content holds
+    # (a small part of the content does not keep a buffer of all of it)
+    return nextoffsets, out[:k] if counted or 2 * k >= size else out[:k].clone()
+
+
 def getitem_inner_range(outer_offsets, inner_offsets, content, start=None, stop=None, step=None):
     """array[..., start:stop:step] of a two-level ListOffsetArray: the outer offsets
     are unchanged; returns (outer_offsets, new inner offsets, new content)."""
-    nextoffsets, nextcarry = inner_range(inner_offsets, start, stop, step)
-    return outer_offsets, nextoffsets, take(content, nextcarry)
+    return (outer_offsets, *range_select(inner_offsets, content, start, stop, step))

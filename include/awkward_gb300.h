@@ -738,12 +738,18 @@ int awkward_ListArray64_getitem_jagged_apply_64_noalloc(int64_t* tooffsets, int6
  *   jagged_index_select: array[index] with a jagged int64 index in one pass
  *     -- jagged_apply with the content gathered at each carry (itemsize 1, 2,
  *     4 or 8; tocarry NULL to skip), errors as jagged_apply's;
+ *   jagged_range_select: array[..., start:stop:step] on one level of lists in
+ *     one pass -- next_range with the content gathered at each carry (itemsize
+ *     1, 2, 4 or 8; absent bounds INT64_MAX); tooffsets[nlists] is the number
+ *     selected, of which the first tolen are written; an element outside
+ *     [0, contentlen) sets err_code to 0 ("index out of range");
  *   take: out[i] = content[carry[i]] for itemsize 1, 2, 4 or 8 bytes
  *     (NumpyArray._carry); a carry outside [0, contentlen) sets err_code to
  *     invocation_index*256 + 0 ("index out of range"). */
 int awkward_gb300_jagged_mask_to_index(int64_t* tooffsets, int64_t* toindex, const uint8_t* mask, const int64_t* offsets, int64_t nlists, uint64_t* err_code, void* stream);
 int awkward_gb300_jagged_mask_select(int64_t* tooffsets, void* tocontent, int64_t* tocarry, const uint8_t* mask, const int64_t* offsets, const void* content, int64_t itemsize, int64_t nlists, uint64_t* err_code, void* stream);
 int awkward_gb300_jagged_index_select(int64_t* tooffsets, void* tocontent, int64_t* tocarry, const int64_t* index_offsets, const int64_t* index, int64_t indexlen, const int64_t* offsets, const void* content, int64_t itemsize, int64_t contentlen, int64_t nlists, uint64_t* err_code, void* stream);
+int awkward_gb300_jagged_range_select(int64_t* tooffsets, void* tocontent, int64_t tolen, const int64_t* offsets, const void* content, int64_t itemsize, int64_t contentlen, int64_t nlists, int64_t start, int64_t stop, int64_t step, uint64_t* err_code, void* stream);
 int awkward_gb300_take(void* out, const void* content, int64_t itemsize, const int64_t* carry, int64_t n, int64_t contentlen, uint64_t invocation_index, uint64_t* err_code, void* stream);
 
 /* ---- backward kernels of differentiable jagged operations (torch.autograd
@@ -805,6 +811,10 @@ int awkward_gb300_reduce_sum_max_argmax_host_float64(double* h_sum, double* h_ma
  * materialised mapped values (sums within the reducers' bound).  Other
  * map or reduce values, or map 1 without y, return cudaErrorInvalidValue. */
 int awkward_gb300_fused_reduce_float64(void* out, const double* x, const double* y, const int64_t* offsets, int64_t nlists, int64_t map, int64_t reduce, uint64_t invocation_index, uint64_t* err_code, void* stream);
+
+/* ---- a few device words to the host (no counterpart in awkward): dst[i] =
+ * *src[i], at most 16 of them, with one wait for the stream. */
+int awkward_gb300_read_words(int64_t* dst, const int64_t* const* src, int64_t n, void* stream);
 
 /* ---- self-test of the failure report (no counterpart in awkward): one warp
  * runs the decoupled look-back of the scan kernels on tile 1 of a fresh
