@@ -75,11 +75,12 @@ __device__ __forceinline__ typename OpOf<K>::type::Out* out_of(const BatchArray&
 }
 
 template <int K, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, kSegMinBlocks * kSegBlock / BLOCK)
+__global__ void __launch_bounds__(BLOCK, kWalkBlocks<typename OpOf<K>::type> * kSegBlock / BLOCK)
     batch_reduce_kernel(typename OpOf<K>::type op, const BatchArray* __restrict__ arrays,
                         const int2* __restrict__ items, const int* __restrict__ order, int nitems,
                         RangeRecord<typename OpOf<K>::type::Acc>* records, unsigned* counter) {
   using Op = typename OpOf<K>::type;
+  __shared__ span_t<Op> span[BLOCK / 32];
   const int lane = threadIdx.x & 31;
   while (true) {
     int k = 0;
@@ -94,7 +95,8 @@ __global__ void __launch_bounds__(BLOCK, kSegMinBlocks * kSegBlock / BLOCK)
     const int Weff = A.ranges[K];
     const long long d0 = D * it.y / Weff, d1 = D * (it.y + 1) / Weff;
     typename Op::Out* out = out_of<K>(A);
-    seg_reduce_range(op, A.x, A.offsets, A.nlists, e0, A.E, d0, d1, out, records[id]);
+    seg_walk(op, A.x, A.offsets, A.nlists, e0, A.E, d0, d1, out, records[id],
+             span[threadIdx.x >> 5]);
     if (lane == 0) records[id].pad = it.x;
   }
 }

@@ -613,61 +613,9 @@ __device__ __forceinline__ FxAcc run_short(const FixedSumOp<IN>& op, const IN* p
   }
 }
 
-// ---------------------------------------------------------------- whole short lists
-// The output of a whole list of n <= kShortList float64 elements at p
-// (global index st) for the lane-per-list rounds of seg_reduce_kernel: the
-// largest raw key in one pass, with nothing but the key kept per element.
-// The raw key is a bijection, so the winner's bits are the key mapped back,
-// and the output equals finalize(run_short(...)) bit for bit whenever *fast
-// stays true -- that is, unless the winner is a zero or a NaN (or, for the
-// arg-reducers, the list starts with a NaN), where the caller reruns
-// run_short's exact path.
-template <bool MAX>
-struct LaneFinal<ExtremumOp<double, MAX>> : std::true_type {};
-template <bool MAX>
-struct LaneFinal<ArgExtremumOp<double, MAX>> : std::true_type {};
-
 // 0 < |b| <= inf: the winner is neither a zero nor a NaN
 __device__ __forceinline__ bool raw_winner_exact(long long b) {
   return (unsigned long long)((b & 0x7fffffffffffffffLL) - 1) < 0x7ff0000000000000ULL;
-}
-
-template <bool MAX>
-__device__ __forceinline__ double lane_final(const ExtremumOp<double, MAX>& op, const double* p,
-                                             int n, long long, bool& fast) {
-  if (n <= 0) return op.ident;
-  const long long* q = reinterpret_cast<const long long*>(p);
-  long long best = kKeyLow;  // the first element is always taken
-  for (int i = 0; i < n; i++) {
-    const long long k = MAX ? f64_raw_key(__ldg(q + i)) : ~f64_raw_key(__ldg(q + i));
-    best = k > best ? k : best;
-  }
-  const long long bits = f64_raw_key(MAX ? best : ~best);  // the raw key is an involution
-  fast = raw_winner_exact(bits);
-  // identity -inf (max) / +inf (min): every non-NaN winner is the output
-  // (an infinite winner equal to the identity has the identity's bits)
-  if (__double_as_longlong(op.ident) == (MAX ? (long long)0xfff0000000000000ULL : 0x7ff0000000000000LL))
-    return __longlong_as_double(bits);
-  return op.finalize({f64_dir_key<MAX>(__longlong_as_double(bits)), bits, 0}, 0);
-}
-
-template <bool MAX>
-__device__ __forceinline__ int64_t lane_final(const ArgExtremumOp<double, MAX>&, const double* p,
-                                              int n, long long st, bool& fast) {
-  if (n <= 0) return -1;
-  const long long* q = reinterpret_cast<const long long*>(p);
-  long long best = kKeyLow;
-  int at = 0;
-  for (int i = 0; i < n; i++) {
-    const long long k = MAX ? f64_raw_key(__ldg(q + i)) : ~f64_raw_key(__ldg(q + i));
-    if (k > best) {
-      best = k;
-      at = i;
-    }
-  }
-  const long long bits = f64_raw_key(MAX ? best : ~best);
-  fast = raw_winner_exact(bits) && !is_nan(__longlong_as_double(__ldg(q)));
-  return st + at;
 }
 
 // ---------------------------------------------------------------- warp runs
@@ -699,6 +647,7 @@ __device__ __forceinline__ typename Op::Acc run_coop_exact(const Op& op,
                                                            long long li) {
   const int sub = threadIdx.x & (G - 1);
   typename Op::Acc a = op.identity();
+#pragma unroll 4
   for (long long j = s + sub; j < e; j += G) a = op.step(a, __ldg(x + j), j, j == st, li);
   return group_allreduce<G>(op, a);
 }
@@ -712,45 +661,63 @@ __device__ typename Op::Acc run_coop(const Op& op, const store_t<typename Op::In
 // Float64 sum: a group-wide largest exponent, then every lane adds its
 // elements aligned to it (one anchor: no renormalisation inside the run, the
 // same truncation whatever the lane order) and the lanes' fixed-point
-// partials are combined.  Runs with an infinity or NaN, or with more than 256
-// elements per lane (a lane partial could exceed 2^62), take the general
-// accumulator.
+// partials are combined.  At most 64 elements per lane are added to one anchor,
+// with two bits kept below its unit (a lane partial stays below 2^62); a longer
+// run is added piece by piece.  A piece with an infinity or NaN takes the
+// general accumulator.
+template <int G>
+__device__ __forceinline__ FxAcc coop_sum_piece(const double* x, long long s, long long e) {
+  const int sub = threadIdx.x & (G - 1);
+  const int* xh = reinterpret_cast<const int*>(x) + 1;
+  int eb = 0;
+#pragma unroll 4
+  for (long long j = s + sub; j < e; j += G) {
+    const int v = __ldg(xh + 2 * j) & 0x7ff00000;
+    eb = v > eb ? v : eb;
+  }
+#pragma unroll
+  for (int d = G / 2; d > 0; d >>= 1) {
+    const int o = __shfl_xor_sync(0xffffffffu, eb, d);
+    eb = o > eb ? o : eb;
+  }
+  const int emax_f = eb >> 20;
+  if (__any_sync(0xffffffffu, emax_f == 0x7ff)) {
+    FxAcc a{0, 1, 0, 0.0};
+    for (long long j = s + sub; j < e; j += G) a = fx_add_f64(a, __ldg(x + j));
+    return a;
+  }
+  const int anchor = emax_f > 1 ? emax_f : 1;
+  const int below = anchor > 2 ? 2 : anchor - 1;
+  const long long* q = reinterpret_cast<const long long*>(x);
+  long long acc = 0;
+#pragma unroll 4
+  for (long long j = s + sub; j < e; j += G) {
+    const long long b = __ldg(q + j);
+    const int ex = (int)((unsigned long long)b >> 52) & 0x7ff;
+    const long long m = (b & 0xfffffffffffffLL) | ((long long)(ex != 0) << 52);
+    const int d = anchor - (ex ? ex : 1);
+    const long long t = (m << below) >> (d < 63 ? d : 63);
+    const long long sg = b >> 63;
+    acc += (t ^ sg) - sg;
+  }
+  return FxAcc{acc, anchor - below, 0, 0.0};
+}
+
 template <int G, class IN>
 __device__ __forceinline__ FxAcc run_coop_sum(const FixedSumOp<IN>& op, const IN* x, long long s,
                                               long long e, long long st, long long li) {
   if constexpr (!std::is_same<IN, double>::value) {
     return run_coop_exact<G>(op, x, s, e, st, li);
   } else {
-    const int sub = threadIdx.x & (G - 1);
-    const int* xh = reinterpret_cast<const int*>(x) + 1;
-    int eb = 0;
-    const bool too_long = e - s > 256ll * G;
-    if (!too_long)
-      for (long long j = s + sub; j < e; j += G) {
-        const int v = __ldg(xh + 2 * j) & 0x7ff00000;
-        eb = v > eb ? v : eb;
-      }
-#pragma unroll
-    for (int d = G / 2; d > 0; d >>= 1) {
-      const int o = __shfl_xor_sync(0xffffffffu, eb, d);
-      eb = o > eb ? o : eb;
+    constexpr long long kPiece = 64ll * G;
+    FxAcc a = coop_sum_piece<G>(x, s, e < s + kPiece ? e : s + kPiece);
+    long long p = s + kPiece;
+    while (__any_sync(0xffffffffu, p < e)) {  // (every group of the warp walks on together)
+      const long long b = p < e ? p : e, c = b + kPiece < e ? b + kPiece : e;
+      a = fx_combine(a, coop_sum_piece<G>(x, b, c));
+      p += kPiece;
     }
-    const int emax_f = eb >> 20;
-    if (__any_sync(0xffffffffu, too_long || emax_f == 0x7ff))
-      return run_coop_exact<G>(op, x, s, e, st, li);
-    const int anchor = emax_f > 1 ? emax_f : 1;
-    const long long* q = reinterpret_cast<const long long*>(x);
-    long long acc = 0;
-    for (long long j = s + sub; j < e; j += G) {
-      const long long b = __ldg(q + j);
-      const int ex = (int)((unsigned long long)b >> 52) & 0x7ff;
-      const long long m = (b & 0xfffffffffffffLL) | ((long long)(ex != 0) << 52);
-      const int d = anchor - (ex ? ex : 1);
-      const long long t = m >> (d < 63 ? d : 63);
-      const long long sg = b >> 63;
-      acc += (t ^ sg) - sg;
-    }
-    return group_allreduce<G>(op, FxAcc{acc, anchor, 0});
+    return group_allreduce<G>(op, a);
   }
 }
 template <int G, class IN>
@@ -772,6 +739,7 @@ __device__ __forceinline__ void raw_group_best(const double* x, long long s, lon
   const int n = (int)(e - s);
   long long best = kKeyLow;
   int at = -1;
+#pragma unroll 4
   for (int j = sub; j < n; j += G) {
     const long long k = MAX ? f64_raw_key(__ldg(q + j)) : ~f64_raw_key(__ldg(q + j));
     if (at < 0 || k > best) {
@@ -890,7 +858,36 @@ struct CenteredSumSqOp {
   __device__ Out finalize(Acc a, long long) const { return a; }
 };
 
+}  // namespace gb
+
+#include "seg_tile.cuh"
+
+namespace gb {
+
 // ---------------------------------------------------------------- launcher
+// The per-array kernel: a persistent grid of warps, each reducing one
+// merge-path range (seg_walk).  The element-parallel walk takes 48 KB of
+// shared memory for its eight warps: four CTAs per SM.
+template <class Op>
+__global__ void __launch_bounds__(kSegBlock, kWalkBlocks<Op>)
+    seg_reduce_kernel(Op op, const store_t<typename Op::In>* __restrict__ x,
+                      const int64_t* __restrict__ offsets, long long nlists,
+                      typename Op::Out* __restrict__ out, RangeRecord<typename Op::Acc>* records,
+                      int W, uint64_t inv, uint64_t* err) {
+  (void)inv;
+  (void)err;
+  __shared__ span_t<Op> span[kSegBlock / 32];
+  const int w = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
+  const long long e0 = __ldg(offsets);
+  const long long eN = __ldg(offsets + nlists);
+  const long long E = eN > e0 ? eN - e0 : 0;
+  const long long D = nlists + E;
+  const int Weff = seg_ranges(nlists, E, W);
+  if (w >= Weff) return;
+  const long long d0 = D * w / Weff, d1 = D * (w + 1) / Weff;
+  seg_walk(op, x, offsets, nlists, e0, E, d0, d1, out, records[w], span[threadIdx.x >> 5]);
+}
+
 template <class Op>
 struct SegReduceConfig {
   static int blocks_per_sm() {

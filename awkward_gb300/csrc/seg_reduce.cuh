@@ -12,21 +12,21 @@
 // range, list I1 is open at its end (the "tail"), and list I0 may have begun
 // in an earlier range (the "head").
 //
-// Reduction.  The warp walks its lists 32 at a time, one list per lane: a
-// list of at most 32 elements is reduced by its lane straight from global
-// memory (read-only path; 64 resident warps per SM keep enough loads in
-// flight, and the warp's loads cover one contiguous stretch of content); a
-// longer list is reduced by the whole warp, strided over 32 lanes (coalesced)
-// and combined with a butterfly.  Each input byte is read from HBM once and
-// results are stored coalesced.
+// Reduction.  Sums and extrema of 4- and 8-byte elements take the
+// element-parallel walk of seg_tile.cuh.  The others walk the warp's lists 32 at
+// a time, one list per lane: a list of at most 32 elements is reduced by its
+// lane straight from global memory (read-only path; the warp's loads cover one
+// contiguous stretch of content); a longer list is reduced by the whole warp,
+// strided over 32 lanes (coalesced) and combined with a butterfly.  Each input
+// byte is read from HBM once and results are stored coalesced.
 //
 // Arithmetic.  Every reducer's combine is commutative and associative
 // (extremum reducers carry the element index and break ties towards the
 // lowest index), so the cooperative reductions give the CPU's results:
 // bit-exact for integers, counts, max/min and argmax/argmin (including the
 // NaN and signed-zero rules).  Float64 data never touch the float64 pipe per
-// element (see reduce_ops.cuh): comparisons use integer keys, sums an exact
-// fixed-point accumulator.
+// element (see seg_tile.cuh, reduce_ops.cuh): comparisons use integer keys,
+// sums an exact fixed-point accumulator.
 //
 // Lists that cross warp ranges leave one head and one tail record per warp;
 // a one-block fix-up kernel combines them with a segmented scan in range
@@ -230,11 +230,6 @@ __device__ __forceinline__ void seg_range_records(const Op& op,
   if (!tail) rec.tail_acc = op.identity();
 }
 
-// The reducers with a direct finisher for a whole list of at most
-// kShortList elements (lane_final, defined with them in reduce_ops.cuh).
-template <class Op>
-struct LaneFinal : std::false_type {};
-
 // Reduce the lists of merge-path diagonal range [d0, d1) of one array (whole
 // warp), writing each list that ends in the range to out[list]; the partials
 // of the giant lists crossing the range ends go to `rec`.
@@ -244,8 +239,7 @@ struct LaneFinal : std::false_type {};
 // below).  A round whose lists all end inside the range with at most
 // kShortList elements each -- nearly every round of short-list data -- is
 // finished by the lanes alone: each computes its list's output with the
-// reducer's short-run arithmetic (lane_final where the reducer has one, else
-// finalize(run_short)) and stores it.  Other rounds (a list longer than
+// reducer's short-run arithmetic and stores it.  Other rounds (a list longer than
 // kShortList, the giant list crossing the range start, the list open at its
 // end) take seg_direct_lists.  Both give the same bits for a list, so the
 // per-array kernel and the batched one (which both call this) agree bit for bit.
@@ -289,12 +283,7 @@ __device__ __forceinline__ void seg_reduce_range(const Op& op,
     const bool plain = li != I1 && (unsigned long long)n <= (unsigned long long)kShortList;
     if (__all_sync(0xffffffffu, !act || plain)) {
       const int m = act ? (int)n : 0;
-      typename Op::Out r;
-      bool fast = true;
-      if constexpr (LaneFinal<Op>::value) r = lane_final(op, x + st, m, st, fast);
-      else r = op.finalize(run_short(op, x + st, m, st, st, li), li);
-      if (!__all_sync(0xffffffffu, fast) && !fast)
-        r = op.finalize(run_short(op, x + st, m, st, st, li), li);
+      const typename Op::Out r = op.finalize(run_short(op, x + st, m, st, st, li), li);
       if (act) out[li] = r;
     } else {
       seg_direct_lists(op, x, base, act, st, en, I1, J0, J1, emit, rec);
@@ -314,27 +303,6 @@ __host__ __device__ __forceinline__ int seg_ranges_min(long long nlists, long lo
 }
 __host__ __device__ __forceinline__ int seg_ranges(long long nlists, long long E, int W) {
   return seg_ranges_min(nlists, E, W, kMinRangeItems);
-}
-
-// The per-array kernel: a persistent grid of warps, each reducing one
-// merge-path range (seg_reduce_range).
-template <class Op>
-__global__ void __launch_bounds__(kSegBlock, kSegMinBlocks)
-    seg_reduce_kernel(Op op, const store_t<typename Op::In>* __restrict__ x,
-                      const int64_t* __restrict__ offsets, long long nlists,
-                      typename Op::Out* __restrict__ out, RangeRecord<typename Op::Acc>* records,
-                      int W, uint64_t inv, uint64_t* err) {
-  (void)inv;
-  (void)err;
-  const int w = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
-  const long long e0 = __ldg(offsets);
-  const long long eN = __ldg(offsets + nlists);
-  const long long E = eN > e0 ? eN - e0 : 0;
-  const long long D = nlists + E;
-  const int Weff = seg_ranges(nlists, E, W);
-  if (w >= Weff) return;
-  const long long d0 = D * w / Weff, d1 = D * (w + 1) / Weff;
-  seg_reduce_range(op, x, offsets, nlists, e0, E, d0, d1, out, records[w]);
 }
 
 // Giant lists (more than kAbsorb elements) that cross warp ranges: one warp
