@@ -23,16 +23,16 @@ CUDA kernels; there is no fallback.
 
 from __future__ import annotations
 
-import numpy as np
+import math
+
 import torch
 
 from . import _abi
-from .kernel_table import backend
+from .kernel_table import raw_stream
 
 DEFAULT_ACTIVATION_BUDGET = 256 * 2**20
 
 _SUFFIX = {torch.float32: "float32", torch.float64: "float64"}
-_NP = {torch.float32: np.float32, torch.float64: np.float64}
 
 
 def _check(values, offsets):
@@ -47,7 +47,7 @@ def _check(values, offsets):
 
 
 def _stream(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return raw_stream(t.device.index)
 
 
 def _launch(name, *args):
@@ -56,12 +56,14 @@ def _launch(name, *args):
         raise RuntimeError(f"{name}: CUDA launch failed with cudaError {rc}")
 
 
-def _reduce(family, out, values, offsets, *extra):
-    dt = _NP[values.dtype]
-    key = {"sum": ("awkward_reduce_sum", dt, dt, np.int64),
-           "max": ("awkward_reduce_max", dt, dt, np.int64),
-           "argmax": ("awkward_reduce_argmax", np.int64, dt, np.int64, np.int64)}[family]
-    backend()[key](out, values, offsets, *extra)
+def _reduce(name, out, values, offsets, *extra):
+    """One of awkward's reducers, straight from the library: it has no error to
+    report, and the kernel table would keep the tensors until the next
+    synchronize()."""
+    rc = _abi.cfunc(name)(out.data_ptr(), values.data_ptr(), offsets.data_ptr(), *extra, 0, None,
+                          _stream(values))
+    if rc != 0:
+        raise RuntimeError(f"{name}: CUDA launch failed with cudaError {rc}")
 
 
 class SegmentSum(torch.autograd.Function):
@@ -70,7 +72,8 @@ class SegmentSum(torch.autograd.Function):
         _check(values, offsets)
         n = offsets.numel() - 1
         out = torch.empty(n, dtype=values.dtype, device=values.device)
-        _reduce("sum", out, values, offsets, n)
+        t = _SUFFIX[values.dtype]
+        _reduce(f"awkward_reduce_sum_{t}_{t}_64", out, values, offsets, n)
         ctx.save_for_backward(offsets)
         ctx.nvalues = values.numel()
         return out
@@ -92,8 +95,9 @@ class SegmentMax(torch.autograd.Function):
         n = offsets.numel() - 1
         out = torch.empty(n, dtype=values.dtype, device=values.device)
         arg = torch.empty(n, dtype=torch.int64, device=values.device)
-        _reduce("max", out, values, offsets, n, -np.inf)
-        _reduce("argmax", arg, values, offsets, offsets[:-1].contiguous(), n)
+        t = _SUFFIX[values.dtype]
+        _reduce(f"awkward_reduce_max_{t}_{t}_64", out, values, offsets, n, -math.inf)
+        _reduce(f"awkward_reduce_argmax_{t}_64", arg, values, offsets, offsets.data_ptr(), n)
         ctx.save_for_backward(arg)
         ctx.nvalues = values.numel()
         return out

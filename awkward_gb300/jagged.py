@@ -26,56 +26,93 @@ Errors follow awkward's protocol and surface as ``ValueError``.
 
 from __future__ import annotations
 
+import threading
+
 import numpy as np
 import torch
 
 from . import _abi
-from .kernel_table import backend
+from ._messages import TIMEOUT_MESSAGE, messages
+from .kernel_table import backend, raw_stream
 
 SLICE_NONE = np.iinfo(np.int64).max  # awkward's kSliceNone
 
 
-def _stream(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
+# Up to this many bytes a result whose size depends on the data is written into
+# a buffer as long as its source, so that no size is read first.
+_WHOLE_SOURCE = 64 << 20
+
+_LOCAL = threading.local()
 
 
-def _err_word(device):
-    return torch.full((1,), -1, dtype=torch.int64, device=device)
+class _Call:
+    """The stream of one call and the thread's error word there.  Every call
+    reads the word back before it returns and leaves it clear, so the next
+    call of the thread on that stream finds it as a new one."""
 
+    def __init__(self, device):
+        index = device.index
+        self.stream = raw_stream(index)
+        words = _LOCAL.__dict__.setdefault("words", {})
+        self.err = words.get((index, self.stream))
+        if self.err is None:
+            if len(words) >= 64:
+                words.clear()
+            self.err = words[index, self.stream] = torch.full((1,), -1, dtype=torch.int64, device=device)
+        self.address = self.err.data_ptr()
 
-def _raise_if(word, what):
-    if word != -1:
-        raise ValueError(f"index out of range in compiled CUDA code ({what})")
+    def finish(self, what, family, *addresses):
+        """The device words at `addresses`; the call's error as ValueError."""
+        *got, word = _abi.read_words(self.stream, *addresses, self.address)
+        if word != -1:
+            self.err.fill_(-1)
+            code = word & 255
+            msg = messages(family)[code] if family else (TIMEOUT_MESSAGE if code else "index out of range")
+            raise ValueError(f"{msg} in compiled CUDA code ({what})")
+        return got
+
+    def span(self, offsets, n, source, itemsize):
+        """Entries to allocate for elements of the lists' span: their number, or
+        `source` (no fewer) when that is small enough."""
+        if n <= 0 or source * itemsize <= _WHOLE_SOURCE:
+            return source if n > 0 else 0
+        first, last = _abi.read_words(self.stream, offsets.data_ptr(), offsets.data_ptr() + 8 * n)
+        return last - first
 
 
 def take(content, carry, check=True):
     """content[carry] (a gather); raises ValueError for a carry outside the content."""
     out = torch.empty(carry.numel(), dtype=content.dtype, device=content.device)
-    err = _err_word(content.device)
+    if check:
+        call = _Call(content.device)
+        stream, address = call.stream, call.address
+    else:
+        unread = torch.full((1,), -1, dtype=torch.int64, device=content.device)
+        stream, address = raw_stream(content.device.index), unread.data_ptr()
     rc = _abi.ext_cfunc("awkward_gb300_take")(
         out.data_ptr(), content.data_ptr(), content.element_size(), carry.data_ptr(),
-        carry.numel(), content.numel(), 0, err.data_ptr(), _stream(content))
+        carry.numel(), content.numel(), 0, address, stream)
     if rc != 0:
         raise RuntimeError(f"awkward_gb300_take: cudaError {rc}")
     if check:
-        _raise_if(int(err.item()), "take")
+        call.finish("take", None)
     return out
 
 
 def jagged_mask_to_index(offsets, mask):
     """(index offsets, local index) of the true entries of a jagged boolean mask."""
     n = offsets.numel() - 1
-    span = int(offsets[-1].item() - offsets[0].item()) if n > 0 else 0
-    tooffsets = torch.empty(n + 1, dtype=torch.int64, device=offsets.device)
-    toindex = torch.empty(max(span, 1), dtype=torch.int64, device=offsets.device)
+    call = _Call(offsets.device)
     m = mask.view(torch.uint8) if mask.dtype == torch.bool else mask
-    err = _err_word(offsets.device)
+    tooffsets = torch.empty(n + 1, dtype=torch.int64, device=offsets.device)
+    toindex = torch.empty(max(call.span(offsets, n, m.numel(), 8), 1), dtype=torch.int64,
+                          device=offsets.device)
     rc = _abi.ext_cfunc("awkward_gb300_jagged_mask_to_index")(
         tooffsets.data_ptr(), toindex.data_ptr(), m.data_ptr(), offsets.data_ptr(), n,
-        err.data_ptr(), _stream(offsets))
+        call.address, call.stream)
     if rc != 0:
         raise RuntimeError(f"awkward_gb300_jagged_mask_to_index: cudaError {rc}")
-    k = int(tooffsets[-1].item())
+    (k,) = call.finish("awkward_gb300_jagged_mask_to_index", None, tooffsets.data_ptr() + 8 * n)
     return tooffsets, toindex[:k]
 
 
@@ -85,19 +122,20 @@ def mask_select(offsets, content, mask, with_carry=False):
     selected element's position in the content) -- the same outputs as
     getitem_jagged_mask without its intermediate local index."""
     n = offsets.numel() - 1
-    span = int(offsets[-1].item() - offsets[0].item()) if n > 0 else 0
-    tooffsets = torch.empty(n + 1, dtype=torch.int64, device=offsets.device)
-    out = torch.empty(max(span, 1), dtype=content.dtype, device=content.device)
-    carry = torch.empty(max(span, 1), dtype=torch.int64, device=offsets.device) if with_carry else None
+    call = _Call(offsets.device)
     m = mask.view(torch.uint8) if mask.dtype == torch.bool else mask
-    err = _err_word(offsets.device)
+    itemsize = content.element_size()
+    span = max(call.span(offsets, n, m.numel(), itemsize + (8 if with_carry else 0)), 1)
+    tooffsets = torch.empty(n + 1, dtype=torch.int64, device=offsets.device)
+    out = torch.empty(span, dtype=content.dtype, device=content.device)
+    carry = torch.empty(span, dtype=torch.int64, device=offsets.device) if with_carry else None
     rc = _abi.ext_cfunc("awkward_gb300_jagged_mask_select")(
         tooffsets.data_ptr(), out.data_ptr(), carry.data_ptr() if with_carry else None,
-        m.data_ptr(), offsets.data_ptr(), content.data_ptr(), content.element_size(), n,
-        err.data_ptr(), _stream(offsets))
+        m.data_ptr(), offsets.data_ptr(), content.data_ptr(), itemsize, n,
+        call.address, call.stream)
     if rc != 0:
         raise RuntimeError(f"awkward_gb300_jagged_mask_select: cudaError {rc}")
-    k = int(tooffsets[-1].item()) if n > 0 else 0
+    (k,) = call.finish("awkward_gb300_jagged_mask_select", None, tooffsets.data_ptr() + 8 * n)
     if with_carry:
         return tooffsets, out[:k], carry[:k]
     return tooffsets, out[:k]
@@ -109,28 +147,23 @@ def index_select(offsets, content, index_offsets, index, with_carry=False):
     content and, with `with_carry`, the carry -- the same outputs as
     getitem_jagged_index without writing and re-reading the carry.  Errors
     are jagged_apply's, raised as ValueError."""
-    from ._messages import messages
-
     n = offsets.numel() - 1
     k = index.numel()
+    call = _Call(offsets.device)
     tooffsets = torch.empty(n + 1, dtype=torch.int64, device=offsets.device)
     out = torch.empty(max(k, 1), dtype=content.dtype, device=content.device)
     carry = torch.empty(max(k, 1), dtype=torch.int64, device=offsets.device) if with_carry else None
     # a one-element stand-in keeps the pointers valid when the content is empty
     src = content if content.numel() > 0 else torch.zeros(1, dtype=content.dtype,
                                                           device=content.device)
-    err = _err_word(offsets.device)
     rc = _abi.ext_cfunc("awkward_gb300_jagged_index_select")(
         tooffsets.data_ptr(), out.data_ptr(), carry.data_ptr() if with_carry else None,
         index_offsets.data_ptr(), index.data_ptr(), k, offsets.data_ptr(), src.data_ptr(),
-        content.element_size(), content.numel(), n, err.data_ptr(), _stream(offsets))
+        content.element_size(), content.numel(), n, call.address, call.stream)
     if rc != 0:
         raise RuntimeError(f"awkward_gb300_jagged_index_select: cudaError {rc}")
-    word = int(err.item()) & ((1 << 64) - 1)
-    if word != (1 << 64) - 1:
-        msg = messages("awkward_ListArray_getitem_jagged_apply")[word & 255]
-        raise ValueError(f"{msg} in compiled CUDA code (awkward_gb300_jagged_index_select)")
-    m = int(tooffsets[-1].item()) if n > 0 else 0
+    (m,) = call.finish("awkward_gb300_jagged_index_select", "awkward_ListArray_getitem_jagged_apply",
+                       tooffsets.data_ptr() + 8 * max(n, 0))
     if with_carry:
         return tooffsets, out[:m], carry[:m]
     return tooffsets, out[:m]
@@ -172,13 +205,13 @@ def inner_range(inner_offsets, start=None, stop=None, step=None):
     be["awkward_ListArray_getitem_next_range_carrylength", np.int64, np.int64, np.int64](
         carrylength, st, sp, n, a, b, c)
     be.synchronize()
-    nextcarry = torch.empty(max(int(carrylength.item()), 1), dtype=torch.int64,
-                            device=inner_offsets.device)
+    length = int(carrylength.item())
+    nextcarry = torch.empty(max(length, 1), dtype=torch.int64, device=inner_offsets.device)
     nextoffsets = torch.empty(n + 1, dtype=torch.int64, device=inner_offsets.device)
     be["awkward_ListArray_getitem_next_range", np.int64, np.int64, np.int64, np.int64](
         nextoffsets, nextcarry, st, sp, n, a, b, c)
     be.synchronize()
-    return nextoffsets, nextcarry[: int(carrylength.item())]
+    return nextoffsets, nextcarry[:length]
 
 
 # Up to this many bytes a selection is written into a buffer as long as the
@@ -195,6 +228,7 @@ def range_select(inner_offsets, content, start=None, stop=None, step=None):
               1 if step is None else step)
     nextoffsets = torch.empty(n + 1, dtype=torch.int64, device=inner_offsets.device)
     size = content.numel()
+    call = _Call(content.device)
     counted = size * content.element_size() > _WHOLE_CONTENT
     if counted:
         be = backend()
@@ -205,15 +239,13 @@ def range_select(inner_offsets, content, start=None, stop=None, step=None):
         size = int(total.item())
     while True:
         out = torch.empty(max(size, 1), dtype=content.dtype, device=content.device)
-        err = _err_word(content.device)
         rc = _abi.ext_cfunc("awkward_gb300_jagged_range_select")(
             nextoffsets.data_ptr(), out.data_ptr(), size, inner_offsets.data_ptr(),
             content.data_ptr(), content.element_size(), content.numel(), n, *bounds,
-            err.data_ptr(), _stream(content))
+            call.address, call.stream)
         if rc != 0:
             raise RuntimeError(f"awkward_gb300_jagged_range_select: cudaError {rc}")
-        k, word = _abi.read_words(_stream(content), nextoffsets.data_ptr() + 8 * n, err.data_ptr())
-        _raise_if(word, "take")
+        (k,) = call.finish("take", None, nextoffsets.data_ptr() + 8 * n)
         if k <= size:
             break
         size = k  # overlapping lists: more selected than the content holds

@@ -96,6 +96,7 @@ class _StreamContext:
 
     def __init__(self, device):
         self.err = torch.full((1,), -1, dtype=torch.int64, device=device)  # NO_ERROR
+        self.address = self.err.data_ptr()
         self.pending = []
 
     def record_error(self, invocation, code, stream):
@@ -104,6 +105,11 @@ class _StreamContext:
         with torch.cuda.stream(stream):
             w = torch.full_like(self.err, word)
             self.err.copy_(torch.where((self.err < 0) | (self.err > w), w, self.err))
+
+
+# The current stream of a device as a raw cudaStream_t (torch.cuda.current_stream
+# builds a Stream object, which costs more than a launch).
+raw_stream = torch._C._cuda_getCurrentRawStream
 
 
 # Device arrays of row pointers (the int64_t** arguments), by device and
@@ -137,61 +143,65 @@ class GB300Kernel:
         self.args = SIGNATURES[name]["args"]
         self.dir = [a[2] for a in self.args]
         self.is_ptr = [a[3] > 0 for a in self.args]
+        # what a call checks, worked out once: pointer depth, dtype, name
+        self._plan = [(a[3], TORCH_OF_C[a[1]], a[0]) for a in self.args]
         self._f = _abi.cfunc(name)
 
     def __repr__(self):
         return f"<GB300Kernel {self.name}>"
 
-    def _convert(self, args):
-        cargs = []
-        keep = []
-        device = None
-        for (an, base, _d, depth, _c, _r), v in zip(self.args, args, strict=True):
-            if depth == 0:
-                cargs.append(v.item() if hasattr(v, "item") else v)
-                continue
-            if depth == 1:
-                t = v
-                if not isinstance(t, torch.Tensor) or not t.is_cuda:
-                    raise TypeError(f"{self.name}: argument {an} must be a CUDA tensor")
-                if t.dtype != TORCH_OF_C[base]:
-                    raise TypeError(f"{self.name}: argument {an} must have dtype "
-                                    f"{TORCH_OF_C[base]}, not {t.dtype}")
-                if not t.is_contiguous():
-                    raise ValueError(f"{self.name}: argument {an} must be contiguous")
-                device = t.device
-                cargs.append(t.data_ptr())
-                keep.append(t)
-                continue
-            rows = list(v)
-            for t in rows:
-                if not isinstance(t, torch.Tensor) or not t.is_cuda or t.dtype != TORCH_OF_C[base]:
-                    raise TypeError(f"{self.name}: rows of {an} must be CUDA {TORCH_OF_C[base]} tensors")
-                device = t.device
-            dev = device if device is not None else torch.device("cuda", torch.cuda.current_device())
-            ptrs = _pointer_array(dev, tuple(t.data_ptr() for t in rows))
-            keep.extend(rows)
-            keep.append(ptrs)
-            cargs.append(ptrs.data_ptr())
-        return cargs, keep, device
+    def _rows(self, an, dtype, v, index):
+        """(pointer array, rows, device index) of a list-of-lists argument."""
+        rows = list(v)
+        for t in rows:
+            if not isinstance(t, torch.Tensor) or not t.is_cuda or t.dtype != dtype:
+                raise TypeError(f"{self.name}: rows of {an} must be CUDA {dtype} tensors")
+            index = t.get_device()
+        dev = torch.device("cuda", torch.cuda.current_device() if index < 0 else index)
+        return _pointer_array(dev, tuple(t.data_ptr() for t in rows)), rows, index
 
     def __call__(self, *args):
-        cargs, keep, device = self._convert(args)
-        if device is None:
-            device = torch.device("cuda", torch.cuda.current_device())
-        stream = torch.cuda.current_stream(device)
-        ctx = self.backend._context(stream)
+        if len(args) != len(self._plan):
+            raise ValueError(f"{self.name}: takes {len(self._plan)} arguments, not {len(args)}")
+        cargs = []
+        keep = []
+        index = -1
+        for (depth, dtype, an), v in zip(self._plan, args):
+            if depth == 0:
+                cargs.append(v.item() if hasattr(v, "item") else v)
+            elif depth == 1:
+                if not isinstance(v, torch.Tensor) or not v.is_cuda:
+                    raise TypeError(f"{self.name}: argument {an} must be a CUDA tensor")
+                if v.dtype is not dtype:
+                    raise TypeError(f"{self.name}: argument {an} must have dtype "
+                                    f"{dtype}, not {v.dtype}")
+                if not v.is_contiguous():
+                    raise ValueError(f"{self.name}: argument {an} must be contiguous")
+                index = v.get_device()
+                cargs.append(v.data_ptr())
+                keep.append(v)
+            else:
+                ptrs, rows, index = self._rows(an, dtype, v, index)
+                keep.extend(rows)
+                keep.append(ptrs)
+                cargs.append(ptrs.data_ptr())
+        if index < 0:
+            index = torch.cuda.current_device()
+        stream = raw_stream(index)
+        ctx = self.backend._context(index, stream)
         if len(ctx.pending) >= MAX_PENDING_INVOCATIONS:
-            self.backend.synchronize(stream)
-            ctx = self.backend._context(stream)
-        invocation = len(ctx.pending)
-        ctx.pending.append(_Invocation(self.family, keep))
-        rc = self._f(*cargs, invocation, ctx.err.data_ptr(), stream.cuda_stream)
+            self.backend.synchronize(torch.cuda.current_stream(index))
+            ctx = self.backend._context(index, stream)
+        pending = ctx.pending
+        invocation = len(pending)
+        pending.append(_Invocation(self.family, keep))
+        rc = self._f(*cargs, invocation, ctx.address, stream)
         if rc != 0:
             raise RuntimeError(f"{self.name}: CUDA launch failed with cudaError {rc}")
-        code = injected_fault(self.name, self.family)
-        if code is not None:
-            ctx.record_error(invocation, code, stream)
+        if FAULT_ENV in os.environ:
+            code = injected_fault(self.name, self.family)
+            if code is not None:
+                ctx.record_error(invocation, code, torch.cuda.current_stream(index))
 
 
 class GB300Backend:
@@ -225,11 +235,11 @@ class GB300Backend:
     def by_name(self, name):
         return self[kernel_key(name)]
 
-    def _context(self, stream):
-        key = (stream.device, stream.cuda_stream)
-        ctx = self._contexts.get(key)
+    def _context(self, index, stream):
+        """The context of raw stream `stream` of device `index`."""
+        ctx = self._contexts.get((index, stream))
         if ctx is None:
-            ctx = self._contexts[key] = _StreamContext(stream.device)
+            ctx = self._contexts[index, stream] = _StreamContext(torch.device("cuda", index))
         return ctx
 
     def selftest_lookback_timeout(self, spin_limit=1000):
@@ -237,29 +247,34 @@ class GB300Backend:
         on the current stream as one more invocation: its wait on a tile that
         never publishes runs out after `spin_limit` polls, so the next
         synchronize() raises the "bounded wait gave up" ValueError."""
-        stream = torch.cuda.current_stream()
-        ctx = self._context(stream)
+        index = torch.cuda.current_device()
+        stream = raw_stream(index)
+        ctx = self._context(index, stream)
         invocation = len(ctx.pending)
         ctx.pending.append(_Invocation("awkward_gb300_selftest_lookback_timeout", []))
         rc = _abi.ext_cfunc("awkward_gb300_selftest_lookback_timeout")(
-            int(spin_limit), invocation, ctx.err.data_ptr(), stream.cuda_stream)
+            int(spin_limit), invocation, ctx.address, stream)
         if rc != 0:
             raise RuntimeError(f"look-back self-test: CUDA launch failed with cudaError {rc}")
 
     def synchronize(self, stream=None):
         """Wait for the stream; raise ValueError for the first failed invocation."""
+        current = torch.cuda.current_stream()
         if stream is None:
-            stream = torch.cuda.current_stream()
-        stream.synchronize()
-        key = (stream.device, stream.cuda_stream)
-        ctx = self._contexts.get(key)
+            stream = current
+        index, raw = stream.device.index, stream.cuda_stream
+        ctx = self._contexts.get((index, raw))
+        if ctx is None or stream != current:
+            stream.synchronize()
         if ctx is None:
             return
+        # reading the word waits for the current stream; without an error the
+        # word is as good as new and the context stays
+        pending, ctx.pending = ctx.pending, []
         word = int(ctx.err.item()) & NO_ERROR
-        pending = ctx.pending
-        self._contexts[key] = _StreamContext(stream.device)
         if word == NO_ERROR:
             return
+        self._contexts[index, raw] = _StreamContext(stream.device)
         inv = pending[word >> ERROR_BITS]
         code = word & ((1 << ERROR_BITS) - 1)
         raise ValueError(f"{messages(inv.name)[code]} in compiled CUDA code ({inv.name})")

@@ -1,0 +1,79 @@
+"""The error words that calls reuse: an error is raised once, by the call it
+belongs to, and the next call on the stream -- or on another stream or thread --
+starts clear; backend().synchronize() keeps a stream's context while there is
+no error and names the right invocation after many error-free ones."""
+
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _select(bad):
+    import torch
+
+    from awkward_gb300 import jagged
+
+    off = torch.tensor([0, 3, 5], dtype=torch.int64, device="cuda")
+    x = torch.arange(5, dtype=torch.float32, device="cuda")
+    ioff = torch.tensor([0, 1, 2], dtype=torch.int64, device="cuda")
+    idx = torch.tensor([2, 7 if bad else -1], dtype=torch.int64, device="cuda")
+    return jagged.index_select(off, x, ioff, idx)[1].tolist()
+
+
+def _alternate():
+    for _ in range(3):
+        with pytest.raises(ValueError, match="index out of range"):
+            _select(True)
+        assert _select(False) == [2.0, 4.0]
+
+
+def test_selection_errors_do_not_stay():
+    import torch
+
+    _alternate()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        _alternate()
+    failed = []
+
+    def work():
+        try:
+            _alternate()
+        except BaseException as e:  # noqa: BLE001
+            failed.append(e)
+
+    threads = [threading.Thread(target=work) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
+
+
+def test_backend_context_survives_error_free_synchronisations():
+    import torch
+
+    import awkward_gb300
+
+    be = awkward_gb300.backend()
+    be.synchronize()
+    off = torch.tensor([0, 3, 5], dtype=torch.int64, device="cuda")
+    x = torch.arange(5, dtype=torch.float64, device="cuda")
+    out = torch.empty(2, dtype=torch.float64, device="cuda")
+    total = be["awkward_reduce_sum", np.float64, np.float64, np.int64]
+    expand = be.by_name("awkward_ListArray64_getitem_jagged_expand_64")
+    i8 = torch.empty(4, dtype=torch.int64, device="cuda")
+    for _ in range(3):
+        for _ in range(2):
+            total(out, x, off, 2)
+            be.synchronize()
+        total(out, x, off, 2)
+        expand(i8, i8.clone(), torch.zeros(3, dtype=torch.int64, device="cuda"), i8.clone(), off[:-1],
+               off[1:], 2, 2)
+        with pytest.raises(ValueError, match=r"cannot fit jagged slice.*getitem_jagged_expand"):
+            be.synchronize()
+    total(out, x, off, 2)
+    be.synchronize()
+    assert out.tolist() == [3.0, 7.0]
