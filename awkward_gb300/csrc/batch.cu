@@ -231,7 +231,7 @@ cudaError_t upload(T** dst, const std::vector<T>& v) {
 //   occupancy_div  persistent CTAs per SM = reducer occupancy / occupancy_div;
 //   range_min      items per reduction range of arrays whose lists all have
 //                  at most kAbsorb elements (any split gives their bits;
-//                  at least kMinRangeItems);
+//                  at least 512);
 //   block          threads per CTA of the reducer launches (128 or 256).
 // err_code: device word for bounded-wait failures of the select scan.
 GB_EXPORT int awkward_gb300_batch_plan_create(
@@ -243,7 +243,7 @@ GB_EXPORT int awkward_gb300_batch_plan_create(
     int64_t order_mode, int64_t occupancy_div, int64_t range_min, int64_t block,
     uint64_t* err_code) {
   *plan = nullptr;
-  if (narrays <= 0 || occupancy_div < 1 || range_min < kMinRangeItems ||
+  if (narrays <= 0 || occupancy_div < 1 || range_min < 512 ||
       (block != 128 && block != 256))
     return (int)cudaErrorInvalidValue;
   Plan* p = new Plan();

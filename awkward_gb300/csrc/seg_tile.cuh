@@ -305,7 +305,8 @@ __device__ __forceinline__ auto word_of(V v) {
 // extremum's identity (nothing beats a NaN identity).
 template <class Op>
 struct WalkState {
-  unsigned low = kRoundLow;  // (never so low that a zero's exponent is in the window)
+  // 2^-16 to 2^9 to begin with (never so low that a zero's exponent is in it)
+  unsigned low = 1023 - 16;
 };
 template <class T, bool MAX>
 struct WalkState<ExtremumOp<T, MAX>> {
