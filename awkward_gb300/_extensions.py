@@ -71,6 +71,8 @@ kernel-specification.yml):
   jagged_mask_select: array[mask] in one pass -- the new offsets, the
     selected content (itemsize 1, 2, 4 or 8) and optionally the carry
     (NULL to skip), without the local index of the chain;
+  jagged_mask_select_sized: the same for a caller who knows the elements in
+    the lists' span, or no fewer (the mask's length);
   jagged_index_select: array[index] with a jagged int64 index in one pass
     -- jagged_apply with the content gathered at each carry (itemsize 1, 2,
     4 or 8; tocarry NULL to skip), errors as jagged_apply's;
@@ -92,6 +94,9 @@ EXTENSIONS["awkward_gb300_jagged_mask_select"] = (
      ("const uint8_t*", "mask"), ("const int64_t*", "offsets"), ("const void*", "content"),
      ("int64_t", "itemsize"), ("int64_t", "nlists"), ("uint64_t*", "err_code"),
      ("void*", "stream")], "jagged")
+EXTENSIONS["awkward_gb300_jagged_mask_select_sized"] = (
+    EXTENSIONS["awkward_gb300_jagged_mask_select"][0][:-2]
+    + [("int64_t", "nelements"), ("uint64_t*", "err_code"), ("void*", "stream")], "jagged")
 EXTENSIONS["awkward_gb300_jagged_index_select"] = (
     [("int64_t*", "tooffsets"), ("void*", "tocontent"), ("int64_t*", "tocarry"),
      ("const int64_t*", "index_offsets"), ("const int64_t*", "index"), ("int64_t", "indexlen"),

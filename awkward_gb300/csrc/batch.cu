@@ -17,11 +17,16 @@
 //
 // Launches per run: 3 x (reducer + fix-up) + select, after 2 memsets; no host
 // synchronisation and no allocation, so a run can be captured in a CUDA graph.
+// Where mask_compact() says so for an array, or from kCompactMin elements in all,
+// select + count goes by the bitmaps of the masks instead (mask_compact.cuh): one
+// launch over the bits tiles of all arrays, whose totals are scanned as one
+// sequence, and one that copies and ranks the list ends.
 #include <algorithm>
 #include <numeric>
 #include <vector>
 
 #include "list_tile.cuh"
+#include "mask_compact.cuh"
 #include "mask_select.cuh"
 #include "reduce_ops.cuh"
 
@@ -40,6 +45,7 @@ struct BatchArray {
   int ranges[kOps];
   int item0[kOps];
   long long tile0;
+  long long mask_tile0;
   double* out_sum;
   double* out_max;
   int64_t* out_argmax;
@@ -169,6 +175,62 @@ __global__ void __launch_bounds__(kTileBlock, 8)
                            A.sel_content, nullptr, A.out_count, st, err);
 }
 
+// The same by the bitmaps of the masks (mask_compact.cuh): tile_array has the array
+// of each bits tile.
+__global__ void __launch_bounds__(kTileBlock)
+    batch_mask_bits_kernel(const BatchArray* __restrict__ arrays,
+                           const int* __restrict__ tile_array, MaskBits b) {
+  __shared__ MaskBitsSmem sm;
+  const BatchArray& A = arrays[tile_array[blockIdx.x]];
+  mask_bits_tile(sm, b, blockIdx.x, blockIdx.x - A.mask_tile0, A.mask,
+                 mask_span(A.mask, A.offsets, A.nlists, A.E));
+}
+
+__global__ void __launch_bounds__(kTileBlock, 4)
+    batch_mask_apply_kernel(const BatchArray* __restrict__ arrays, int narrays,
+                            const int* __restrict__ tile_array, long long mask_tiles,
+                            const long long* __restrict__ tile_base, long long ntiles, MaskBits b,
+                            unsigned copy_blocks) {
+  if (blockIdx.x < copy_blocks) {
+    const long long chunks = mask_tiles * (kMaskTile / kChunk);
+    const long long step = (long long)copy_blocks * (kTileBlock / 32);
+    long long c = (blockIdx.x * (long long)kTileBlock + threadIdx.x) >> 5;
+    if (c >= chunks) return;
+    MaskChunk next = mask_chunk(b, c);
+    for (; c < chunks; c += step) {
+      const MaskChunk ch = next;
+      if (c + step < chunks) next = mask_chunk(b, c + step);
+      if (!__any_sync(0xffffffffu, ch.word != 0u)) continue;
+      const BatchArray& A = arrays[tile_array[c / (kMaskTile / kChunk)]];
+      const MaskSpan span = mask_span(A.mask, A.offsets, A.nlists, A.E);
+      const long long e0 = span.first - span.shift +
+                           (c - A.mask_tile0 * (kMaskTile / kChunk)) * kChunk + (threadIdx.x & 31);
+      mask_copy<double, false>(ch, A.x + e0,
+                               A.sel_content + (ch.tile_before - b.tile_before[A.mask_tile0]),
+                               nullptr, e0);
+    }
+    return;
+  }
+  for (long long g = blockIdx.x - copy_blocks; g < ntiles; g += gridDim.x - copy_blocks) {
+    int lo = 0, hi = narrays;  // last array with tile_base <= g
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (tile_base[mid] <= g) lo = mid;
+      else hi = mid;
+    }
+    const BatchArray& A = arrays[lo];
+    const MaskSpan span = mask_span(A.mask, A.offsets, A.nlists, A.E);
+    const long long before = b.tile_before[A.mask_tile0];
+    const long long l0 = (g - A.tile0) * kTileLists;
+    for (long long l = l0 + threadIdx.x; l < l0 + kTileLists && l < A.nlists; l += kTileBlock) {
+      const long long o = __ldg(A.offsets + l), end = __ldg(A.offsets + l + 1);
+      A.sel_offsets[l] = mask_rank(o, b, A.mask_tile0, span) - before;
+      A.out_count[l] = end - o;
+      if (l + 1 == A.nlists) A.sel_offsets[l + 1] = mask_rank(end, b, A.mask_tile0, span) - before;
+    }
+  }
+}
+
 struct Plan {
   int narrays = 0;
   int block = kSegBlock;  // threads per CTA of the reducer launches
@@ -182,6 +244,9 @@ struct Plan {
   unsigned* d_counters = nullptr;          // one per reducer
   unsigned long long* d_scan = nullptr;    // select ticket + tile states
   long long* d_tile_base = nullptr;
+  long long mask_tiles = 0;                // 0: batch_select_kernel
+  int* d_tile_array = nullptr;
+  void* d_mask_bits = nullptr;
   uint64_t* err = nullptr;
 };
 
@@ -210,6 +275,8 @@ void free_plan(Plan* p) {
   cudaFree(p->d_counters);
   cudaFree(p->d_scan);
   cudaFree(p->d_tile_base);
+  cudaFree(p->d_tile_array);
+  cudaFree(p->d_mask_bits);
   delete p;
 }
 
@@ -259,6 +326,9 @@ GB_EXPORT int awkward_gb300_batch_plan_create(
   std::vector<BatchArray> arrays(narrays);
   std::vector<std::vector<int2>> items(kOps);
   std::vector<long long> tile_base(narrays + 1, 0);
+  std::vector<int> tile_array;
+  long long elements = 0;
+  bool compact = false;
   for (int a = 0; a < narrays; a++) {
     BatchArray& A = arrays[a];
     A.x = x[a];
@@ -279,6 +349,10 @@ GB_EXPORT int awkward_gb300_batch_plan_create(
       A.item0[k] = (int)items[k].size();
       for (int w = 0; w < A.ranges[k]; w++) items[k].push_back(make_int2(a, w));
     }
+    A.mask_tile0 = (long long)tile_array.size();
+    if (nlists[a] > 0) tile_array.insert(tile_array.end(), mask_tiles(A.E), a);
+    elements += A.E;
+    compact |= nlists[a] > 0 && mask_compact(A.E, nlists[a]);
     A.tile0 = tile_base[a];
     tile_base[a + 1] = tile_base[a] + (nlists[a] > 0 ? tile_count(nlists[a]) : 0);
     A.out_sum = out_sum[a];
@@ -318,6 +392,13 @@ GB_EXPORT int awkward_gb300_batch_plan_create(
   if (e != cudaSuccess) {
     free_plan(p);
     return (int)e;
+  }
+  if (compact || elements >= kCompactMin) {
+    const long long tiles = (long long)tile_array.size();
+    e = upload(&p->d_tile_array, tile_array);
+    if (e == cudaSuccess) e = cudaMalloc(&p->d_mask_bits, mask_bits_bytes(tiles));
+    if (e == cudaSuccess) p->mask_tiles = tiles;
+    else cudaGetLastError();  // no room for the bitmaps: batch_select_kernel needs none
   }
   *plan = p;
   return 0;
@@ -375,7 +456,20 @@ GB_EXPORT int awkward_gb300_batch_plan_run(void* plan, void* stream) {
     batch_fixup_kernel<2><<<(p->nitems[2] + 255) / 256, 256, 0, s>>>(
         op2, p->d_arrays, static_cast<RangeRecord<ArgOpD::Acc>*>(p->d_records[2]), p->nitems[2]);
   }
-  if (p->ntiles > 0) {
+  if (p->mask_tiles > 0) {
+    const MaskBits b = mask_bits_at(p->d_mask_bits, p->mask_tiles);
+    e = cudaMemsetAsync(b.finished, 0, sizeof(*b.finished), s);
+    if (e != cudaSuccess) return (int)e;
+    batch_mask_bits_kernel<<<(unsigned)p->mask_tiles, kTileBlock, 0, s>>>(p->d_arrays,
+                                                                          p->d_tile_array, b);
+    const long long most = device_sm_count() * 4;
+    const long long copies = p->mask_tiles * (kMaskTile / kChunk) / (kTileBlock / 32);
+    const unsigned nc = (unsigned)std::min(copies, most);
+    const unsigned nl = (unsigned)std::min(p->ntiles, most);
+    batch_mask_apply_kernel<<<nc + nl, kTileBlock, 0, s>>>(p->d_arrays, p->narrays, p->d_tile_array,
+                                                           p->mask_tiles, p->d_tile_base, p->ntiles,
+                                                           b, nc);
+  } else if (p->ntiles > 0) {
     batch_select_kernel<<<(unsigned)p->ntiles, kTileBlock, 0, s>>>(
         p->d_arrays, p->narrays, p->d_tile_base, p->d_scan, p->d_scan + 1, p->err);
   }

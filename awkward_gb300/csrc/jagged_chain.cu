@@ -19,6 +19,7 @@
 // prefix and writing the local index (position within its list) of each at
 // its rank.
 #include "list_tile.cuh"
+#include "mask_compact.cuh"
 #include "mask_select.cuh"
 
 using namespace gb;
@@ -213,6 +214,42 @@ __global__ void __launch_bounds__(kTileBlock, 8)
                       nullptr, st, err);
 }
 
+// array[mask] by the bitmap of the whole mask (mask_compact.cuh).
+__global__ void __launch_bounds__(kTileBlock)
+    mask_bits_kernel(MaskBits b, const uint8_t* __restrict__ mask, const int64_t* __restrict__ offsets,
+                     long long nlists, long long nelements) {
+  __shared__ MaskBitsSmem sm;
+  mask_bits_tile(sm, b, blockIdx.x, blockIdx.x, mask, mask_span(mask, offsets, nlists, nelements));
+}
+
+template <class W, bool CARRY>
+__global__ void __launch_bounds__(kTileBlock, 4)
+    mask_apply_kernel(MaskBits b, const uint8_t* __restrict__ mask, const int64_t* __restrict__ offsets,
+                      long long nlists, long long nelements, const W* __restrict__ content,
+                      int64_t* __restrict__ tooffsets, W* __restrict__ tocontent,
+                      int64_t* __restrict__ tocarry, unsigned copy_blocks) {
+  const MaskSpan span = mask_span(mask, offsets, nlists, nelements);
+  if (blockIdx.x < copy_blocks) {
+    const long long used = (span.nbits + kChunk - 1) / kChunk;
+    const long long step = (long long)copy_blocks * (kTileBlock / 32);
+    long long c = (blockIdx.x * (long long)kTileBlock + threadIdx.x) >> 5;
+    if (c >= used) return;
+    MaskChunk next = mask_chunk(b, c);
+    for (; c < used; c += step) {
+      const MaskChunk ch = next;
+      if (c + step < used) next = mask_chunk(b, c + step);
+      const long long e0 = span.first - span.shift + c * kChunk + (threadIdx.x & 31);
+      mask_copy<W, CARRY>(ch, content + e0, tocontent + ch.tile_before,
+                          CARRY ? tocarry + ch.tile_before : nullptr, e0);
+    }
+    return;
+  }
+  const long long blocks = gridDim.x - copy_blocks;
+  for (long long i = (blockIdx.x - copy_blocks) * (long long)kTileBlock + threadIdx.x; i <= nlists;
+       i += blocks * kTileBlock)
+    tooffsets[i] = mask_rank(__ldg(offsets + i), b, 0, span);
+}
+
 }  // namespace
 
 // The new offsets (nlists + 1 entries) and, for each true entry of the mask
@@ -313,5 +350,54 @@ GB_EXPORT int awkward_gb300_jagged_mask_select(int64_t* tooffsets, void* toconte
   }
   e = cudaGetLastError();
   cudaError_t f = scratch_free(scratch, s);
+  return (int)(e != cudaSuccess ? e : f);
+}
+
+// The same with the number of elements in the lists' span, or a bound for it
+// (the mask's length), at hand: where mask_compact() says so the call goes by the
+// bitmap of the whole mask.
+GB_EXPORT int awkward_gb300_jagged_mask_select_sized(int64_t* tooffsets, void* tocontent,
+                                                     int64_t* tocarry, const uint8_t* mask,
+                                                     const int64_t* offsets, const void* content,
+                                                     int64_t itemsize, int64_t nlists,
+                                                     int64_t nelements, uint64_t* err_code,
+                                                     void* stream) {
+  if (nlists <= 0 || !mask_compact(nelements, nlists))
+    return awkward_gb300_jagged_mask_select(tooffsets, tocontent, tocarry, mask, offsets, content,
+                                            itemsize, nlists, err_code, stream);
+  if (itemsize != 1 && itemsize != 2 && itemsize != 4 && itemsize != 8)
+    return (int)cudaErrorInvalidValue;
+  cudaStream_t s = (cudaStream_t)stream;
+  const long long tiles = mask_tiles(nelements);
+  void* tables = nullptr;
+  if (scratch_alloc(&tables, mask_bits_bytes(tiles), s) != cudaSuccess) {
+    cudaGetLastError();  // no room for the bitmap: the other way needs none
+    return awkward_gb300_jagged_mask_select(tooffsets, tocontent, tocarry, mask, offsets, content,
+                                            itemsize, nlists, err_code, stream);
+  }
+  const MaskBits b = mask_bits_at(tables, tiles);
+  cudaError_t e = cudaMemsetAsync(b.finished, 0, sizeof(*b.finished), s);
+  if (e == cudaSuccess) {
+    mask_bits_kernel<<<(unsigned)tiles, kTileBlock, 0, s>>>(b, mask, offsets, nlists, nelements);
+    const long long sms = device_sm_count();
+    const long long copies = tiles * (kMaskTile / kChunk) / (kTileBlock / 32);
+    const long long lists = (nlists + kTileBlock) / kTileBlock;
+    const unsigned nc = (unsigned)(copies < sms * 4 ? copies : sms * 4);
+    const unsigned nl = (unsigned)(lists < sms * 4 ? lists : sms * 4);
+#define GB_MASK_APPLY(W)                                                                       \
+  (tocarry ? mask_apply_kernel<W, true> : mask_apply_kernel<W, false>)<<<nc + nl, kTileBlock,  \
+                                                                        0, s>>>(               \
+      b, mask, offsets, nlists, nelements, (const W*)content, tooffsets, (W*)tocontent,        \
+      tocarry, nc)
+    switch (itemsize) {
+      case 1: GB_MASK_APPLY(uint8_t); break;
+      case 2: GB_MASK_APPLY(uint16_t); break;
+      case 4: GB_MASK_APPLY(uint32_t); break;
+      default: GB_MASK_APPLY(uint64_t);
+    }
+#undef GB_MASK_APPLY
+    e = cudaGetLastError();
+  }
+  cudaError_t f = scratch_free(tables, s);
   return (int)(e != cudaSuccess ? e : f);
 }

@@ -117,7 +117,7 @@ def jagged_mask_to_index(offsets, mask):
 
 
 def mask_select(offsets, content, mask, with_carry=False):
-    """array[mask] in one pass (awkward_gb300_jagged_mask_select): the new
+    """array[mask] at once (awkward_gb300_jagged_mask_select_sized): the new
     offsets, the selected content and, with `with_carry`, the carry (each
     selected element's position in the content) -- the same outputs as
     getitem_jagged_mask without its intermediate local index."""
@@ -129,12 +129,12 @@ def mask_select(offsets, content, mask, with_carry=False):
     tooffsets = torch.empty(n + 1, dtype=torch.int64, device=offsets.device)
     out = torch.empty(span, dtype=content.dtype, device=content.device)
     carry = torch.empty(span, dtype=torch.int64, device=offsets.device) if with_carry else None
-    rc = _abi.ext_cfunc("awkward_gb300_jagged_mask_select")(
+    rc = _abi.ext_cfunc("awkward_gb300_jagged_mask_select_sized")(
         tooffsets.data_ptr(), out.data_ptr(), carry.data_ptr() if with_carry else None,
-        m.data_ptr(), offsets.data_ptr(), content.data_ptr(), itemsize, n,
+        m.data_ptr(), offsets.data_ptr(), content.data_ptr(), itemsize, n, span,
         call.address, call.stream)
     if rc != 0:
-        raise RuntimeError(f"awkward_gb300_jagged_mask_select: cudaError {rc}")
+        raise RuntimeError(f"awkward_gb300_jagged_mask_select_sized: cudaError {rc}")
     (k,) = call.finish("awkward_gb300_jagged_mask_select", None, tooffsets.data_ptr() + 8 * n)
     if with_carry:
         return tooffsets, out[:k], carry[:k]
