@@ -9,17 +9,8 @@
 //                      d x_j = y_j (g_j - sum_k g_k y_k)         (fused Jacobian product)
 // The forward sum and max use the segmented reducers of this library.
 //
-// Layout: a CTA owns a tile of kSoftLists consecutive lists, one statistics
-// thread per list, and twice as many threads for the memory passes.  It stages
-// the tile's offsets and, when the tile's elements fit
-// (kSoftBytes per array), the element arrays it reads more than once in
-// shared memory by asynchronous copies (cp.async, issued from the tile's two
-// end offsets so they are in flight with the offsets loads), plus an
-// element -> list map (one byte per element).  Per-list statistics (max, sums) are computed by one thread
-// per list in element order, from shared memory; then the tile's elements are
-// visited with consecutive threads on consecutive elements, so every global
-// read and write is coalesced.  A tile whose elements do not fit reads them
-// from global memory and finds each element's list by binary search.
+// The sum's and float softmax kernels work in rounds of 32 lists per warp, without
+// block barriers.
 #include <math.h>
 
 #include "list_tile.cuh"
@@ -38,84 +29,18 @@ __device__ __forceinline__ double exp_t<double>(double v) { return exp(v); }
 template <class T>
 __device__ __forceinline__ T max_t(T a, T b) { return a > b ? a : b; }
 
-constexpr int kSoftLists = 64;        // lists per CTA (one statistics thread each)
-constexpr int kSoftThreads = 128;     // threads per CTA (staging and element passes)
-constexpr int kSoftBytes = 8192;      // staging per element array
-constexpr int kSoftElems = 2048;      // element -> list map entries (>= kSoftBytes / 4)
-
-struct SoftTile {
-  long long loc[kSoftLists + 1];  // offsets of the tile's lists, relative to its first element
-  unsigned char owner[kSoftElems];
-  long long base;                 // first element of the tile
-  int count;                      // lists in this tile
-  int mapped;                     // owner[] holds every element's list
-};
-
-// One element global -> shared memory without a register round trip
-// (cp.async, completed by cp_async_wait_all).
+// Zero a[j] for j outside [offsets[0], offsets[nlists]) within [0, nvalues): the
+// elements no list covers, by threads t of `stride`.  Only those elements are
+// touched (none when the offsets span the whole array).
 template <class T>
-__device__ __forceinline__ void cp_async_elem(T* dst, const T* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(sizeof(T))
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_all;" ::: "memory");
-}
-
-// Stage a tile: offsets[l0 .. l0+count] and, if the tile has at most `cap`
-// elements, its elements of src0 (and src1 when given) into dst0 (dst1) and
-// the element -> list map (all threads; ends with __syncthreads).  The
-// element copies are issued first, from the tile's two end offsets alone, so
-// they are in flight together with the offsets loads.
-template <class T>
-__device__ __forceinline__ void stage_soft_tile(SoftTile& t, const int64_t* __restrict__ offsets,
-                                                long long l0, long long nlists, int cap,
-                                                T* dst0, const T* __restrict__ src0, T* dst1,
-                                                const T* __restrict__ src1) {
-  const long long rem = nlists - l0;
-  const int count = (int)(rem < kSoftLists ? rem : kSoftLists);
-  const long long base = __ldg(offsets + l0);
-  const long long total = __ldg(offsets + l0 + count) - base;
-  const bool mapped = total <= cap;
-  if (mapped) {
-    for (long long q = threadIdx.x; q < total; q += blockDim.x) {
-      cp_async_elem(dst0 + q, src0 + base + q);
-      if (src1) cp_async_elem(dst1 + q, src1 + base + q);
-    }
-  }
-  for (int i = threadIdx.x; i <= kSoftLists; i += blockDim.x) {
-    const int k = i < count ? i : count;
-    t.loc[i] = __ldg(offsets + l0 + k) - base;
-  }
-  if (threadIdx.x == 0) {
-    t.base = base;
-    t.count = count;
-    t.mapped = mapped ? 1 : 0;
-  }
-  __syncthreads();
-  if (mapped && (int)threadIdx.x < count) {
-    const int a = (int)t.loc[threadIdx.x], b = (int)t.loc[threadIdx.x + 1];
-    for (int q = a; q < b; q++) t.owner[q] = (unsigned char)threadIdx.x;
-  }
-  cp_async_wait_all();
-  __syncthreads();
-}
-
-// List of tile element q: the map, or the last r with loc[r] <= q.
-__device__ __forceinline__ int soft_list(const SoftTile& t, long long q) {
-  if (t.mapped) return t.owner[q];
-  int lo = 0, hi = t.count;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (t.loc[mid] <= q) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-
-inline unsigned soft_tiles(long long nlists) {
-  return (unsigned)((nlists + kSoftLists - 1) / kSoftLists);
+__device__ __forceinline__ void zero_outside(T* __restrict__ a, const int64_t* __restrict__ offsets,
+                                             long long nlists, long long nvalues, long long t,
+                                             long long stride) {
+  long long lo = __ldg(offsets), hi = __ldg(offsets + nlists);
+  lo = lo < 0 ? 0 : (lo > nvalues ? nvalues : lo);
+  hi = hi < lo ? lo : (hi > nvalues ? nvalues : hi);
+  for (long long j = t; j < lo; j += stride) a[j] = T(0);
+  for (long long j = hi + t; j < nvalues; j += stride) a[j] = T(0);
 }
 
 // ---------------------------------------------------------------- sum backward
@@ -130,7 +55,10 @@ constexpr int kBcastStage = 1024;  // elements staged per warp and round
 template <class T>
 __global__ void __launch_bounds__(256)
     sum_backward_rounds_kernel(T* __restrict__ gx, const T* __restrict__ gout,
-                               const int64_t* __restrict__ offsets, long long nlists) {
+                               const int64_t* __restrict__ offsets, long long nlists,
+                               long long nvalues) {
+  zero_outside(gx, offsets, nlists, nvalues, blockIdx.x * (long long)blockDim.x + threadIdx.x,
+               (long long)gridDim.x * blockDim.x);
   __shared__ T stage[256 / 32][kBcastStage];
   T* sw = stage[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
@@ -176,115 +104,387 @@ __global__ void max_backward_kernel(T* __restrict__ gx, const T* __restrict__ go
 }
 
 // ---------------------------------------------------------------- softmax
+// Floats go by rounds of 32 lists, one per warp, a list's bounds on each lane.  The round's
+// longest list chooses how many lanes share a list, 4 to 32, and how many elements
+// a lane has, 6 at most; these are loaded once, kept in registers, reduced with
+// shuffles among the list's lanes and stored, the loads of several steps in flight.
+// A round with a list of more than kSoftLongest elements goes list by list, a warp
+// on each, in three passes.  Bound by the instructions of places past the lists' ends
+// at first, by HBM from mean 16 on: 1M lists, us (forward, backward with y kept):
+// mean 4 44, 43 -> 21, 21; mean 16 61, 68 -> 36, 46 (128 and 192 MB, 19 and 28 us);
+// 20000 lists of mean 500 188, 425 -> 113, 208.  Before, tiles of 64 lists were
+// staged in shared memory, one thread reducing each list.
+constexpr int kSoftThreads = 128;
+constexpr int kSoftLongest = 32 * 6;
+constexpr int kSoftFlight = 24;  // 4-byte words a lane has in flight
+
+template <class T, class F>
+__device__ __forceinline__ T lanes_reduce(T v, int lanes, F f) {
+  for (int d = 1; d < lanes; d <<= 1) v = f(v, __shfl_xor_sync(0xffffffffu, v, d));
+  return v;
+}
 template <class T>
-__global__ void __launch_bounds__(kSoftThreads)
-    softmax_forward_kernel(T* __restrict__ y, const T* __restrict__ x,
-                           const int64_t* __restrict__ offsets, long long nlists) {
-  constexpr int cap = kSoftBytes / (int)sizeof(T);
-  __shared__ SoftTile t;
-  __shared__ T sx[cap];
-  __shared__ T s_max[kSoftLists];
-  __shared__ T s_sum[kSoftLists];
-  const long long l0 = (long long)blockIdx.x * kSoftLists;
-  stage_soft_tile(t, offsets, l0, nlists, cap, sx, x, (T*)nullptr, (const T*)nullptr);
-  const long long total = t.loc[t.count];
-  const T* xs = t.mapped ? sx : x + t.base;
-  const int r = threadIdx.x;
-  if (r < t.count) {  // per-list max and sum of exp(x - max)
-    const long long a = t.loc[r], b = t.loc[r + 1];
+__device__ __forceinline__ T lanes_max(T v, int lanes) {
+  return lanes_reduce(v, lanes, [](T a, T b) { return max_t(a, b); });
+}
+template <class T>
+__device__ __forceinline__ T lanes_sum(T v, int lanes) {
+  return lanes_reduce(v, lanes, [](T a, T b) { return a + b; });
+}
+
+// What becomes of a list whose elements a lane group holds: in[0] = x (forward), or
+// in[0] = gy and in[1] = the saved y or x (backward).
+struct SoftForward {
+  static constexpr int kArrays = 1;
+  static constexpr bool kZeroPad = false;
+  template <class T, int N>
+  __device__ __forceinline__ static void apply(const T (&in)[1][N], T (&out)[N], int lanes) {
     T m = -INFINITY;
-    for (long long q = a; q < b; q++) m = max_t(m, xs[q]);
+#pragma unroll
+    for (int k = 0; k < N; k++) m = max_t(m, in[0][k]);
+    m = lanes_max(m, lanes);
     T sum = 0;
-    for (long long q = a; q < b; q++) sum += exp_t(xs[q] - m);
-    s_max[r] = m;
-    s_sum[r] = T(1) / sum;  // one division per list; elements multiply by it
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+      out[k] = exp_t(in[0][k] - m);
+      sum += out[k];
+    }
+    const T inv = T(1) / lanes_sum(sum, lanes);  // one division per list; elements multiply by it
+#pragma unroll
+    for (int k = 0; k < N; k++) out[k] *= inv;
   }
-  __syncthreads();
-  for (long long q = threadIdx.x; q < total; q += blockDim.x) {
-    const int l = soft_list(t, q);
-    y[t.base + q] = exp_t(xs[q] - s_max[l]) * s_sum[l];
+  // one list by a warp: x[0 .. n)
+  template <class T>
+  __device__ __forceinline__ static void list(T* out, const T* const (&in)[1], long long n, int lane) {
+    T m = -INFINITY, sum = 0;
+    for (long long q = lane; q < n; q += 32) m = max_t(m, in[0][q]);
+    m = lanes_max(m, 32);
+    for (long long q = lane; q < n; q += 32) sum += out[q] = exp_t(in[0][q] - m);
+    const T inv = T(1) / lanes_sum(sum, 32);
+    for (long long q = lane; q < n; q += 32) out[q] *= inv;
+  }
+};
+// d x_j = y_j (g_j - sum_k g_k y_k)
+struct SoftBackwardSaved {
+  static constexpr int kArrays = 2;
+  static constexpr bool kZeroPad = true;
+  template <class T, int N>
+  __device__ __forceinline__ static void apply(const T (&in)[2][N], T (&out)[N], int lanes) {
+    T dot = 0;
+#pragma unroll
+    for (int k = 0; k < N; k++) dot += in[0][k] * in[1][k];
+    dot = lanes_sum(dot, lanes);
+#pragma unroll
+    for (int k = 0; k < N; k++) out[k] = in[1][k] * (in[0][k] - dot);
+  }
+  template <class T>
+  __device__ __forceinline__ static void list(T* out, const T* const (&in)[2], long long n, int lane) {
+    T dot = 0;
+    for (long long q = lane; q < n; q += 32) dot += in[0][q] * in[1][q];
+    dot = lanes_sum(dot, 32);
+    for (long long q = lane; q < n; q += 32) out[q] = in[1][q] * (in[0][q] - dot);
+  }
+};
+// The same with y computed again from x.
+struct SoftBackward {
+  static constexpr int kArrays = 2;
+  static constexpr bool kZeroPad = false;
+  template <class T, int N>
+  __device__ __forceinline__ static void apply(const T (&in)[2][N], T (&out)[N], int lanes) {
+    T m = -INFINITY;
+#pragma unroll
+    for (int k = 0; k < N; k++) m = max_t(m, in[1][k]);
+    m = lanes_max(m, lanes);
+    T sum = 0, gsum = 0;
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+      out[k] = exp_t(in[1][k] - m);
+      sum += out[k];
+      gsum += in[0][k] * out[k];
+    }
+    const T inv = T(1) / lanes_sum(sum, lanes);
+    const T dot = lanes_sum(gsum, lanes) * inv;
+#pragma unroll
+    for (int k = 0; k < N; k++) out[k] = out[k] * inv * (in[0][k] - dot);
+  }
+  template <class T>
+  __device__ __forceinline__ static void list(T* out, const T* const (&in)[2], long long n, int lane) {
+    T m = -INFINITY, sum = 0, gsum = 0;
+    for (long long q = lane; q < n; q += 32) m = max_t(m, in[1][q]);
+    m = lanes_max(m, 32);
+    for (long long q = lane; q < n; q += 32) {
+      const T e = out[q] = exp_t(in[1][q] - m);
+      sum += e;
+      gsum += in[0][q] * e;
+    }
+    const T inv = T(1) / lanes_sum(sum, 32);
+    const T dot = lanes_sum(gsum, 32) * inv;
+    for (long long q = lane; q < n; q += 32)
+      out[q] = out[q] * inv * (in[0][q] - dot);
+  }
+};
+
+// One round whose lists have at most LANES * ITEMS elements: lane l holds list l's
+// first element (relative to the pointers) and length.
+template <int LANES, int ITEMS, class Op, class T>
+__device__ __forceinline__ void soft_round(Op, T* __restrict__ out, const T* const (&in)[Op::kArrays],
+                                           int first, int len, int lane) {
+  constexpr int kMost = kSoftFlight / ((int)sizeof(T) / 4 * ITEMS * Op::kArrays);
+  constexpr int kSteps = kMost >= 4 ? 4 : kMost >= 2 ? 2 : 1;  // steps in flight
+  const int i0 = lane % LANES;
+#pragma unroll 1
+  for (int s0 = 0; s0 < LANES; s0 += kSteps) {
+    T v[kSteps][Op::kArrays][ITEMS];
+    int at[kSteps], left[kSteps];  // the lane's first element, the elements from there on
+#pragma unroll
+    for (int s = 0; s < kSteps; s++) {
+      const int from = (s0 + s) * (32 / LANES) + lane / LANES;
+      at[s] = __shfl_sync(0xffffffffu, first, from) + i0;
+      left[s] = __shfl_sync(0xffffffffu, len, from) - i0;
+#pragma unroll
+      for (int k = 0; k < ITEMS; k++)
+#pragma unroll
+        for (int a = 0; a < Op::kArrays; a++)
+          v[s][a][k] = k * LANES < left[s] ? __ldg(in[a] + at[s] + k * LANES)
+                       : a == Op::kArrays - 1 && !Op::kZeroPad ? T(-INFINITY) : T(0);
+    }
+#pragma unroll
+    for (int s = 0; s < kSteps; s++) {
+      T r[ITEMS];
+      Op::apply(v[s], r, LANES);
+#pragma unroll
+      for (int k = 0; k < ITEMS; k++)
+        if (k * LANES < left[s]) out[at[s] + k * LANES] = r[k];
+    }
   }
 }
 
-// d x_j = y_j (g_j - sum_k g_k y_k); y from `ysaved` when given, else
-// recomputed from x (max and normaliser recomputed per list).
-template <class T>
+template <class Op>
 __global__ void __launch_bounds__(kSoftThreads)
-    softmax_backward_kernel(T* __restrict__ gx, const T* __restrict__ gy,
-                            const T* __restrict__ x, const T* __restrict__ ysaved,
-                            const int64_t* __restrict__ offsets, long long nlists) {
-  constexpr int cap = kSoftBytes / (int)sizeof(T);
-  __shared__ SoftTile t;
-  __shared__ T sa[cap];  // x, or the saved y
-  __shared__ T sg[cap];  // gy
-  __shared__ T s_max[kSoftLists];
-  __shared__ T s_sum[kSoftLists];
-  __shared__ T s_dot[kSoftLists];
-  const long long l0 = (long long)blockIdx.x * kSoftLists;
-  const T* src = ysaved ? ysaved : x;
-  stage_soft_tile(t, offsets, l0, nlists, cap, sa, src, sg, gy);
-  const long long total = t.loc[t.count];
-  const T* as = t.mapped ? sa : src + t.base;
-  const T* gs = t.mapped ? sg : gy + t.base;
-  const int r = threadIdx.x;
-  if (ysaved) {
-    if (r < t.count) {
-      const long long a = t.loc[r], b = t.loc[r + 1];
-      T d = 0;
-      for (long long q = a; q < b; q++) d += gs[q] * as[q];
-      s_dot[r] = d;
-    }
-    __syncthreads();
-    for (long long q = threadIdx.x; q < total; q += blockDim.x) {
-      const int l = soft_list(t, q);
-      gx[t.base + q] = as[q] * (gs[q] - s_dot[l]);
+    softmax_kernel(float* __restrict__ out, const float* __restrict__ in0, const float* __restrict__ in1,
+                   const int64_t* __restrict__ offsets, long long nlists, long long nvalues,
+                   unsigned rounds_blocks) {
+  if (blockIdx.x >= rounds_blocks) {  // the elements no list covers
+    zero_outside(out, offsets, nlists, nvalues,
+                 (blockIdx.x - rounds_blocks) * (long long)kSoftThreads + threadIdx.x,
+                 (long long)(gridDim.x - rounds_blocks) * kSoftThreads);
+    return;
+  }
+  const int lane = threadIdx.x & 31;
+  const long long l0 = (blockIdx.x * (long long)(kSoftThreads / 32) + (threadIdx.x >> 5)) * 32;
+  if (l0 >= nlists) return;
+  const long long l = l0 + lane;
+  const long long begin = __ldg(offsets + (l < nlists ? l : nlists));
+  const long long end = __ldg(offsets + (l < nlists ? l + 1 : nlists));
+  const long long base = __shfl_sync(0xffffffffu, begin, 0);
+  const long long n = end - begin;
+  const float* const in[2] = {in0, in1};
+  if (__any_sync(0xffffffffu, n < 0 || n > kSoftLongest)) {
+    for (int j = 0; j < 32; j++) {
+      const long long b = __shfl_sync(0xffffffffu, begin, j), m = __shfl_sync(0xffffffffu, n, j);
+      const float* p[Op::kArrays];
+#pragma unroll
+      for (int a = 0; a < Op::kArrays; a++) p[a] = in[a] + b;
+      if (m > 0) Op::list(out + b, p, m, lane);
     }
     return;
   }
-  if (r < t.count) {
-    const long long a = t.loc[r], b = t.loc[r + 1];
-    T m = -INFINITY;
-    for (long long q = a; q < b; q++) m = max_t(m, as[q]);
-    T sum = 0, gsum = 0;
-    for (long long q = a; q < b; q++) {
-      const T e = exp_t(as[q] - m);
-      sum += e;
-      gsum += gs[q] * e;
+  const float* p[Op::kArrays];
+#pragma unroll
+  for (int a = 0; a < Op::kArrays; a++) p[a] = in[a] + base;
+  const int first = (int)(begin - base), len = (int)n;
+  const int longest = __reduce_max_sync(0xffffffffu, len);
+  float* o = out + base;
+  if (longest <= 8) soft_round<4, 2>(Op(), o, p, first, len, lane);
+  else if (longest <= 16) soft_round<4, 4>(Op(), o, p, first, len, lane);
+  else if (longest <= 24) soft_round<4, 6>(Op(), o, p, first, len, lane);
+  else if (longest <= 32) soft_round<8, 4>(Op(), o, p, first, len, lane);
+  else if (longest <= 48) soft_round<8, 6>(Op(), o, p, first, len, lane);
+  else if (longest <= 96) soft_round<16, 6>(Op(), o, p, first, len, lane);
+  else soft_round<32, 6>(Op(), o, p, first, len, lane);
+}
+
+// Doubles, whose exponentials and sums fill the narrow 64-bit unit, go by tiles of
+// kTileSoft lists per CTA instead, where no lane works for a place past a list's
+// end: the tile's elements are staged in shared memory with a map from elements to
+// lists, the list's threads reduce it, and all threads take the elements, one
+// exponential each.  A tile of more elements goes list by list.
+// 1M lists, us (forward, backward with y kept, with y computed again): mean 4
+// 502, 64, 498 -> 220, 54, 265; mean 16 1390, 149, 1475 -> 689, 146, 826; mean 24,
+// whose tiles of 64 lists did not fit, 1987, 234, 2103 -> 969, 193, 1152 (the kernel
+// for floats: 590, 93, 674; 1275, 203, 1459; 1975, 306, 2265).
+constexpr int kTileSoft = 64;
+constexpr int kTileElems = 1024;
+
+struct SoftTile {
+  long long loc[kTileSoft + 1];  // offsets of the tile's lists, relative to its first element
+  unsigned char owner[kTileElems];  // list of each element
+  long long base;                 // first element of the tile
+  int count;                      // lists in this tile
+  int mapped;                     // the elements fit
+};
+
+// One element global -> shared memory without a register round trip
+// (cp.async, completed by cp_async_wait_all).
+template <class T>
+__device__ __forceinline__ void cp_async_elem(T* dst, const T* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(sizeof(T))
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// Stage a tile of `lists` lists: offsets[l0 .. l0+count] and, if it has at most
+// kTileElems elements, its elements of src0 (and src1 when given) into dst0 (dst1) and
+// the element -> list map (all threads; ends with __syncthreads).  The
+// element copies are issued first, from the tile's two end offsets alone, so
+// they are in flight together with the offsets loads.
+template <class T>
+__device__ __forceinline__ void stage_soft_tile(SoftTile& t, const int64_t* __restrict__ offsets,
+                                                long long l0, long long nlists, int lists, T* dst0, const T* __restrict__ src0, T* dst1,
+                                                const T* __restrict__ src1) {
+  const long long rem = nlists - l0;
+  const int count = (int)(rem < lists ? rem : lists);
+  const long long base = __ldg(offsets + l0);
+  const long long total = __ldg(offsets + l0 + count) - base;
+  const bool mapped = total <= kTileElems;
+  if (mapped) {
+    for (long long q = threadIdx.x; q < total; q += blockDim.x) {
+      cp_async_elem(dst0 + q, src0 + base + q);
+      if (src1) cp_async_elem(dst1 + q, src1 + base + q);
     }
-    s_max[r] = m;
-    const T inv = T(1) / sum;  // one division per list; elements multiply by it
-    s_sum[r] = inv;
-    s_dot[r] = gsum * inv;
+  }
+  for (int i = threadIdx.x; i <= kTileSoft; i += blockDim.x) {
+    const int k = i < count ? i : count;
+    t.loc[i] = __ldg(offsets + l0 + k) - base;
+  }
+  if (threadIdx.x == 0) {
+    t.base = base;
+    t.count = count;
+    t.mapped = mapped ? 1 : 0;
   }
   __syncthreads();
-  for (long long q = threadIdx.x; q < total; q += blockDim.x) {
-    const int l = soft_list(t, q);
-    const T yj = exp_t(as[q] - s_max[l]) * s_sum[l];
-    gx[t.base + q] = yj * (gs[q] - s_dot[l]);
+  if (mapped && (int)threadIdx.x < count) {
+    const int a = (int)t.loc[threadIdx.x], b = (int)t.loc[threadIdx.x + 1];
+    for (int q = a; q < b; q++) t.owner[q] = (unsigned char)threadIdx.x;
+  }
+  cp_async_wait_all();
+  __syncthreads();
+}
+
+// A thread's share of its list: kSoftThreads / lists threads, of one warp, for each.
+struct SoftShare {
+  int list, begin, end, step;
+};
+__device__ __forceinline__ SoftShare soft_share(const SoftTile& t, int lists) {
+  const int step = kSoftThreads / lists, r = threadIdx.x / step;
+  if (r >= t.count) return {r, 0, 0, step};
+  return {r, (int)t.loc[r] + (int)threadIdx.x % step, (int)t.loc[r + 1], step};
+}
+
+// s_list[] and s_dot[] have a place for each list of the tile, also past its last.
+__device__ __forceinline__ void soft_tile(SoftForward, const SoftTile& t, int lists, double* s0,
+                                          const double*, double* s_list, double*,
+                                          double* __restrict__ out) {
+  const SoftShare h = soft_share(t, lists);
+  const int total = (int)t.loc[t.count];
+  double m = -INFINITY;
+  for (int q = h.begin; q < h.end; q += h.step) m = max_t(m, s0[q]);
+  s_list[h.list] = lanes_max(m, h.step);
+  __syncthreads();
+  for (int q = threadIdx.x; q < total; q += kSoftThreads) s0[q] = exp_t(s0[q] - s_list[t.owner[q]]);
+  __syncthreads();
+  double sum = 0;
+  for (int q = h.begin; q < h.end; q += h.step) sum += s0[q];
+  s_list[h.list] = 1.0 / lanes_sum(sum, h.step);
+  __syncthreads();
+  for (int q = threadIdx.x; q < total; q += kSoftThreads) out[q] = s0[q] * s_list[t.owner[q]];
+}
+__device__ __forceinline__ void soft_tile(SoftBackwardSaved, const SoftTile& t, int lists, double* sg,
+                                          const double* sy, double* s_list, double*,
+                                          double* __restrict__ out) {
+  const SoftShare h = soft_share(t, lists);
+  const int total = (int)t.loc[t.count];
+  double d = 0;
+  for (int q = h.begin; q < h.end; q += h.step) d += sg[q] * sy[q];
+  s_list[h.list] = lanes_sum(d, h.step);
+  __syncthreads();
+  for (int q = threadIdx.x; q < total; q += kSoftThreads)
+    out[q] = sy[q] * (sg[q] - s_list[t.owner[q]]);
+}
+__device__ __forceinline__ void soft_tile(SoftBackward, const SoftTile& t, int lists, double* sg,
+                                          double* sx, double* s_list, double* s_dot,
+                                          double* __restrict__ out) {
+  const SoftShare h = soft_share(t, lists);
+  const int total = (int)t.loc[t.count];
+  double m = -INFINITY;
+  for (int q = h.begin; q < h.end; q += h.step) m = max_t(m, sx[q]);
+  s_list[h.list] = lanes_max(m, h.step);
+  __syncthreads();
+  for (int q = threadIdx.x; q < total; q += kSoftThreads) sx[q] = exp_t(sx[q] - s_list[t.owner[q]]);
+  __syncthreads();
+  double sum = 0, gsum = 0;
+  for (int q = h.begin; q < h.end; q += h.step) {
+    sum += sx[q];
+    gsum += sg[q] * sx[q];
+  }
+  const double inv = 1.0 / lanes_sum(sum, h.step);
+  s_list[h.list] = inv;
+  s_dot[h.list] = lanes_sum(gsum, h.step) * inv;
+  __syncthreads();
+  for (int q = threadIdx.x; q < total; q += kSoftThreads) {
+    const int l = t.owner[q];
+    out[q] = sx[q] * s_list[l] * (sg[q] - s_dot[l]);
   }
 }
 
-// Zero a[j] for j outside [offsets[0], offsets[nlists]) within [0, nvalues):
-// the elements no list covers, which the kernels above never write.  Only
-// those elements are touched (none when the offsets span the whole array),
-// so the callers need not clear the whole output first.
-template <class T>
-__global__ void zero_outside_kernel(T* __restrict__ a, const int64_t* __restrict__ offsets,
-                                    long long nlists, long long nvalues) {
-  long long lo = __ldg(offsets), hi = __ldg(offsets + nlists);
-  lo = lo < 0 ? 0 : (lo > nvalues ? nvalues : lo);
-  hi = hi < lo ? lo : (hi > nvalues ? nvalues : hi);
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  for (long long j = t; j < lo; j += stride) a[j] = T(0);
-  for (long long j = hi + t; j < nvalues; j += stride) a[j] = T(0);
+template <class Op>
+__global__ void __launch_bounds__(kSoftThreads)
+    softmax_tile_kernel(double* __restrict__ out, const double* __restrict__ in0,
+                        const double* __restrict__ in1, const int64_t* __restrict__ offsets,
+                        long long nlists, long long nvalues, int lists, unsigned tiles) {
+  __shared__ SoftTile t;
+  __shared__ double s0[kTileElems], s1[Op::kArrays == 2 ? kTileElems : 1];
+  __shared__ double s_list[kTileSoft], s_dot[kTileSoft];
+  if (blockIdx.x >= tiles) {
+    zero_outside(out, offsets, nlists, nvalues,
+                 (blockIdx.x - tiles) * (long long)kSoftThreads + threadIdx.x,
+                 (long long)(gridDim.x - tiles) * kSoftThreads);
+    return;
+  }
+  stage_soft_tile(t, offsets, (long long)blockIdx.x * lists, nlists, lists, s0, in0,
+                  Op::kArrays == 2 ? s1 : nullptr, Op::kArrays == 2 ? in1 : nullptr);
+  if (t.mapped) {
+    soft_tile(Op(), t, lists, s0, s1, s_list, s_dot, out + t.base);
+    return;
+  }
+  const double* const in[2] = {in0, in1};
+  for (int r = threadIdx.x >> 5; r < t.count; r += kSoftThreads / 32) {
+    const double* p[Op::kArrays];
+#pragma unroll
+    for (int a = 0; a < Op::kArrays; a++) p[a] = in[a] + t.base + t.loc[r];
+    Op::list(out + t.base + t.loc[r], p, t.loc[r + 1] - t.loc[r], threadIdx.x & 31);
+  }
 }
 
-template <class T>
-cudaError_t zero_outside(T* a, const int64_t* offsets, long long nlists, long long nvalues,
-                         cudaStream_t s) {
-  if (nvalues <= 0) return cudaSuccess;
-  zero_outside_kernel<T><<<device_sm_count() * 4, 256, 0, s>>>(a, offsets, nlists, nvalues);
+template <class Op, class T>
+cudaError_t softmax(T* out, const T* in0, const T* in1, const int64_t* offsets, long long nlists,
+                    long long nvalues, cudaStream_t s) {
+  // doubles: the most lists, 8 to kTileSoft, of which a tile's elements fit with a
+  // quarter to spare (by the mean length)
+  int lists = sizeof(T) == 8 ? kTileSoft : kSoftThreads;
+  if (sizeof(T) == 8)
+    while (lists > 8 && nvalues / nlists * lists > kTileElems / 5 * 4) lists /= 2;
+  const unsigned blocks = (unsigned)((nlists + lists - 1) / lists);
+  const unsigned rest = nvalues > 0 ? 2 * device_sm_count() : 0;
+  if constexpr (sizeof(T) == 8)
+    softmax_tile_kernel<Op><<<blocks + rest, kSoftThreads, 0, s>>>(out, in0, in1, offsets, nlists,
+                                                                   nvalues, lists, blocks);
+  else
+    softmax_kernel<Op><<<blocks + rest, kSoftThreads, 0, s>>>(out, in0, in1, offsets, nlists,
+                                                              nvalues, blocks);
   return cudaGetLastError();
 }
 
@@ -297,10 +497,9 @@ cudaError_t zero_outside(T* a, const int64_t* offsets, long long nlists, long lo
       void* stream) {                                                                           \
     cudaStream_t s = (cudaStream_t)stream;                                                      \
     if (nlists <= 0) return (int)(nvalues > 0 ? cudaMemsetAsync(grad_x, 0, sizeof(T) * (size_t)nvalues, s) : cudaSuccess); \
-    sum_backward_rounds_kernel<T><<<device_sm_count() * 8, 256, 0, s>>>(grad_x, grad_out,    \
-                                                                       offsets, nlists);        \
-    cudaError_t e = cudaGetLastError();                                                         \
-    return (int)(e != cudaSuccess ? e : zero_outside(grad_x, offsets, nlists, nvalues, s));     \
+    sum_backward_rounds_kernel<T><<<device_sm_count() * 8, 256, 0, s>>>(                        \
+        grad_x, grad_out, offsets, nlists, nvalues);                                            \
+    return (int)cudaGetLastError();                                                             \
   }                                                                                             \
   GB_EXPORT int awkward_gb300_segment_max_backward_##SUFFIX(                                    \
       T* grad_x, const T* grad_out, const int64_t* argmax, int64_t nelements, int64_t nlists,  \
@@ -321,19 +520,17 @@ cudaError_t zero_outside(T* a, const int64_t* offsets, long long nlists, long lo
       T* y, const T* x, const int64_t* offsets, int64_t nlists, int64_t nvalues, void* stream) { \
     cudaStream_t s = (cudaStream_t)stream;                                                      \
     if (nlists <= 0) return (int)(nvalues > 0 ? cudaMemsetAsync(y, 0, sizeof(T) * (size_t)nvalues, s) : cudaSuccess); \
-    softmax_forward_kernel<T><<<soft_tiles(nlists), kSoftThreads, 0, s>>>(y, x, offsets, nlists); \
-    cudaError_t e = cudaGetLastError();                                                         \
-    return (int)(e != cudaSuccess ? e : zero_outside(y, offsets, nlists, nvalues, s));          \
+    return (int)softmax<SoftForward, T>(y, x, (const T*)nullptr, offsets, nlists, nvalues, s);  \
   }                                                                                             \
   GB_EXPORT int awkward_gb300_jagged_softmax_backward_##SUFFIX(                                 \
       T* grad_x, const T* grad_y, const T* x, const T* y_saved, const int64_t* offsets,        \
       int64_t nlists, int64_t nvalues, void* stream) {                                          \
     cudaStream_t s = (cudaStream_t)stream;                                                      \
     if (nlists <= 0) return (int)(nvalues > 0 ? cudaMemsetAsync(grad_x, 0, sizeof(T) * (size_t)nvalues, s) : cudaSuccess); \
-    softmax_backward_kernel<T><<<soft_tiles(nlists), kSoftThreads, 0, s>>>(                    \
-        grad_x, grad_y, x, y_saved, offsets, nlists);                                           \
-    cudaError_t e = cudaGetLastError();                                                         \
-    return (int)(e != cudaSuccess ? e : zero_outside(grad_x, offsets, nlists, nvalues, s));     \
+    return (int)(y_saved ? softmax<SoftBackwardSaved, T>(grad_x, grad_y, y_saved, offsets,      \
+                                                         nlists, nvalues, s)                    \
+                         : softmax<SoftBackward, T>(grad_x, grad_y, x, offsets, nlists,         \
+                                                    nvalues, s));                               \
   }
 
 GB_AUTOGRAD(float32, float)
