@@ -176,10 +176,11 @@ __device__ __forceinline__ double fx_fixed_value(FxAcc a) {
 
 __device__ __forceinline__ double fx_finalize(FxAcc a) { return fx_fixed_value(a) + a.dp; }
 
-// Sum of float64 (or float32) into float64 on the integer pipe in fixed
-// point, rounded once at the end (runs of at most 32 elements also add half
-// their elements in float64, see run_short); within n*eps*sum|x| of the exact
-// sum, like the CPU loop that rounds after every addition.
+// Sum of float64 (or float32) into float64, rounded once at the end: float64 by
+// the exact sums of the tile walk (seg_tile.cuh) where its window holds the
+// elements, else on the integer pipe in fixed point (mapped short runs also add
+// half their elements in float64, see run_short); within n*eps*sum|x| of the
+// exact sum, like the CPU loop that rounds after every addition.
 template <class IN>
 struct FixedSumOp {
   using In = IN;
@@ -430,32 +431,17 @@ struct ArgExtremumOp<double, MAX> {
   __device__ Out finalize(Acc a, long long) const { return a.idx; }
 };
 
-// Put the later cache sectors of a short run in flight before its loop walks
-// them (loads whose results are never read: nothing waits for them, so the
-// misses overlap instead of following one another).
-#pragma nv_diag_suppress 550  // the touch loads' destination is never read, by design
-__device__ __forceinline__ void touch_run(const void* p, int n, int esize) {
-  const char* c = reinterpret_cast<const char*>(p);
-  long long d;
-  if (n > 4) asm volatile("ld.global.nc.b64 %0, [%1];" : "=l"(d) : "l"(c + 4 * esize));
-  if (n > 8) asm volatile("ld.global.nc.b64 %0, [%1];" : "=l"(d) : "l"(c + 8 * esize));
-  if (n > 12) asm volatile("ld.global.nc.b64 %0, [%1];" : "=l"(d) : "l"(c + 12 * esize));
-}
-#pragma nv_diag_default 550
-
 // ---------------------------------------------------------------- short runs
 // Element loaders of the short-run reducers: global memory through the
-// read-only path (with "touch" loads that put a run's later sectors in
-// flight), or a run staged in shared memory.  Both give the same arithmetic.
+// read-only path, or a run staged in shared memory (the double reducers below
+// take only these: their lists in global memory go by the tile walk).
 struct LdGlobal {
-  static constexpr bool kTouch = true;
   template <class T>
   __device__ __forceinline__ T operator()(const T* p) const {
     return __ldg(p);
   }
 };
 struct LdShared {
-  static constexpr bool kTouch = false;
   template <class T>
   __device__ __forceinline__ T operator()(const T* p) const {
     return *p;
@@ -493,7 +479,6 @@ template <bool MAX, class Ld = LdGlobal>
 __device__ __forceinline__ typename ExtremumOp<double, MAX>::Acc run_short(
     const ExtremumOp<double, MAX>& op, const double* p, int n, long long j0, long long st,
     long long li, Ld ld = Ld{}) {
-  if constexpr (Ld::kTouch) touch_run(p, n, 8);
   const long long* q = reinterpret_cast<const long long*>(p);
   long long best = 0;
   int at = -1;
@@ -552,8 +537,7 @@ __device__ __forceinline__ FxAcc run_short(const FixedSumOp<IN>& op, const IN* p
     // pipes; the float64 partial rides in FxAcc::dp and is added to the
     // rounded fixed-point part at the end (IEEE inf/NaN included).  The
     // result stays within n*eps*sum|x| of the exact sum.
-    if constexpr (Ld::kTouch) touch_run(p, n, 8);
-    const long long* q = reinterpret_cast<const long long*>(p);
+      const long long* q = reinterpret_cast<const long long*>(p);
     const int* qh = reinterpret_cast<const int*>(p) + 1;
     double dsum = 0.0;
     int ebmax = 0, ebmin = 0x7ff00000;
