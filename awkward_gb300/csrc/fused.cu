@@ -8,7 +8,7 @@
 // and nothing is written but the per-list results.
 //
 // Maps: x, x*y, x*x, |x| (products rounded once, as an elementwise kernel
-// rounds them).  Reductions: sum (the fixed-point sum of the reducers), max,
+// rounds them).  Reductions: sum (in fixed point, rounded once), max,
 // min (identity -inf / +inf), argmax, argmin (global element indices, -1 for
 // empty lists) -- each equal to materialising the mapped values and calling
 // awkward_reduce_* on them: bit for bit for max/min/argmax/argmin, and within

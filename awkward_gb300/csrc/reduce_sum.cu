@@ -13,7 +13,7 @@ using namespace gb;
                                   (cudaStream_t)stream);                                       \
   }
 
-// float64 results of floating inputs: exact fixed-point accumulation (no
+// float64 results of floating inputs: exact or fixed-point accumulation (no
 // per-element float64 arithmetic)
 #define GB_FSUM(NAME, IN)                                                                      \
   GB_EXPORT int NAME(double* toptr, const IN* fromptr, const int64_t* offsets, int64_t outlength, \

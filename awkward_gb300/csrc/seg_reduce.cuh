@@ -26,7 +26,7 @@
 // bit-exact for integers, counts, max/min and argmax/argmin (including the
 // NaN and signed-zero rules).  Float64 data never touch the float64 pipe per
 // element (see seg_tile.cuh, reduce_ops.cuh): comparisons use integer keys,
-// sums an exact fixed-point accumulator.
+// sums integer accumulators.
 //
 // Lists that cross warp ranges leave one head and one tail record per warp;
 // a one-block fix-up kernel combines them with a segmented scan in range

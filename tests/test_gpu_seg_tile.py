@@ -135,3 +135,23 @@ def test_exact_sums(lengths, how):
         else:
             size = np.array([math.fsum(abs(x[a:b])) for a, b in zip(off, off[1:])])
             assert (abs(got - exact) <= np.maximum(L, 1) * np.finfo(np.float64).eps * size).all()
+
+
+@pytest.mark.parametrize("n", [545, 767, 800, 4096, 4097, 70_000, 300_001])
+@pytest.mark.parametrize("shift", SHIFTS)
+def test_float32_sums_of_long_runs(n, shift):
+    """A lane's chain has an eighth of its elements: at most n/256 + 1 additions, three
+    inside a block of eight, five between lanes and the partials of at most n/256
+    ranges, 32 at a time with five between lanes."""
+    import torch
+
+    rng = np.random.default_rng(n)
+    off = np.array([0, 2, 2 + n, 2 + n, 7 + n], dtype=np.int64) + shift
+    x = (rng.standard_normal(int(off[-1])) + 1).astype(np.float32)
+    out = torch.empty(4, dtype=torch.float32, device="cuda")
+    got = _call("awkward_reduce_sum_float32_float32_64",
+                (torch.from_numpy(x).cuda(), torch.from_numpy(off).cuda(), 4), out)
+    for i in range(4):
+        part = x[off[i]:off[i + 1]].astype(np.float64)
+        k = n / 256 + n / 8192 + 24
+        assert abs(float(got[i]) - math.fsum(part)) <= 1.01 * k * 2.0**-24 * abs(part).sum()
