@@ -10,8 +10,8 @@ kernels, for CUDA tensors:
   and the content carried (``NumpyArray._carry``);
 * ``getitem_jagged_index`` -- ``array[idx]`` with a jagged int64 index
   (same apply + carry); ``index_select`` does it in one kernel (the apply
-  with the content gathered at each carry), ``mask_select`` the same for
-  ``array[mask]``;
+  with the content gathered at each carry), ``mask_select`` does
+  ``array[mask]`` without the local index;
 * ``getitem_inner_range``  -- ``array[..., start:stop:step]`` on the innermost
   list level of a two-level ListOffsetArray, in one kernel (``range_select``);
   ``inner_range`` and ``take`` are awkward's own steps:
