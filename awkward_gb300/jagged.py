@@ -80,6 +80,15 @@ class _Call:
         return last - first
 
 
+def _array(name, t, dtype=None):
+    """`t` as the library reads it: a contiguous CUDA tensor, of `dtype` if that is given."""
+    if not isinstance(t, torch.Tensor) or not t.is_cuda:
+        raise TypeError(f"{name} must be a CUDA tensor")
+    if dtype is not None and t.dtype is not dtype:
+        raise TypeError(f"{name} must have dtype {dtype}, not {t.dtype}")
+    return t.contiguous()
+
+
 def take(content, carry, check=True):
     """content[carry] (a gather); raises ValueError for a carry outside the content."""
     out = torch.empty(carry.numel(), dtype=content.dtype, device=content.device)
@@ -222,7 +231,10 @@ _WHOLE_CONTENT = 1 << 30
 def range_select(inner_offsets, content, start=None, stop=None, step=None):
     """(nextoffsets, selected content) of [start:stop:step] on every list of one
     level in one pass (awkward_gb300_jagged_range_select): inner_range and take
-    without writing and re-reading the carry."""
+    without writing and re-reading the carry.  Offsets are checked as the kernel
+    table checks them (TypeError unless CUDA int64), strided ones made contiguous."""
+    inner_offsets = _array("inner_offsets", inner_offsets, torch.int64)
+    content = _array("content", content)
     n = inner_offsets.numel() - 1
     bounds = (SLICE_NONE if start is None else start, SLICE_NONE if stop is None else stop,
               1 if step is None else step)
