@@ -73,6 +73,9 @@ kernel-specification.yml):
     (NULL to skip), without the local index of the chain;
   jagged_mask_select_sized: the same for a caller who knows the elements in
     the lists' span, or no fewer (the mask's length);
+  jagged_mask_to_index_within, jagged_mask_select_within: the same for a mask
+    of known length -- lists that reach outside its masklen entries set
+    err_code to 0 ("index out of range") and none outside is read;
   jagged_index_select: array[index] with a jagged int64 index in one pass
     -- jagged_apply with the content gathered at each carry (itemsize 1, 2,
     4 or 8; tocarry NULL to skip), errors as jagged_apply's;
@@ -97,6 +100,12 @@ EXTENSIONS["awkward_gb300_jagged_mask_select"] = (
 EXTENSIONS["awkward_gb300_jagged_mask_select_sized"] = (
     EXTENSIONS["awkward_gb300_jagged_mask_select"][0][:-2]
     + [("int64_t", "nelements"), ("uint64_t*", "err_code"), ("void*", "stream")], "jagged")
+EXTENSIONS["awkward_gb300_jagged_mask_to_index_within"] = (
+    EXTENSIONS["awkward_gb300_jagged_mask_to_index"][0][:3] + [("int64_t", "masklen")]
+    + EXTENSIONS["awkward_gb300_jagged_mask_to_index"][0][3:], "jagged")
+EXTENSIONS["awkward_gb300_jagged_mask_select_within"] = (
+    EXTENSIONS["awkward_gb300_jagged_mask_select_sized"][0][:4] + [("int64_t", "masklen")]
+    + EXTENSIONS["awkward_gb300_jagged_mask_select_sized"][0][4:], "jagged")
 EXTENSIONS["awkward_gb300_jagged_index_select"] = (
     [("int64_t*", "tooffsets"), ("void*", "tocontent"), ("int64_t*", "tocarry"),
      ("const int64_t*", "index_offsets"), ("const int64_t*", "index"), ("int64_t", "indexlen"),

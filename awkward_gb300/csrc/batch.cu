@@ -171,8 +171,8 @@ __global__ void __launch_bounds__(kTileBlock, 8)
   ScanTiles st;
   st.ticket = ticket;
   st.status = status + A.tile0;
-  mask_select_tile<double>(sm, tile, A.nlists, A.offsets, A.mask, A.x, A.sel_offsets,
-                           A.sel_content, nullptr, A.out_count, st, err);
+  mask_select_tile<double>(sm, tile, A.nlists, A.offsets, A.mask, kAnyLength, A.x,
+                           A.sel_offsets, A.sel_content, nullptr, A.out_count, st, err);
 }
 
 // The same by the bitmaps of the masks (mask_compact.cuh): tile_array has the array
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(kTileBlock)
   __shared__ MaskBitsSmem sm;
   const BatchArray& A = arrays[tile_array[blockIdx.x]];
   mask_bits_tile(sm, b, blockIdx.x, blockIdx.x - A.mask_tile0, A.mask,
-                 mask_span(A.mask, A.offsets, A.nlists, A.E));
+                 mask_span(A.mask, kAnyLength, A.offsets, A.nlists, A.E));
 }
 
 __global__ void __launch_bounds__(kTileBlock, 4)
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kTileBlock, 4)
       if (c + step < chunks) next = mask_chunk(b, c + step);
       if (!__any_sync(0xffffffffu, ch.word != 0u)) continue;
       const BatchArray& A = arrays[tile_array[c / (kMaskTile / kChunk)]];
-      const MaskSpan span = mask_span(A.mask, A.offsets, A.nlists, A.E);
+      const MaskSpan span = mask_span(A.mask, kAnyLength, A.offsets, A.nlists, A.E);
       const long long e0 = span.first - span.shift +
                            (c - A.mask_tile0 * (kMaskTile / kChunk)) * kChunk + (threadIdx.x & 31);
       mask_copy<double, false>(ch, A.x + e0,
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kTileBlock, 4)
       else hi = mid;
     }
     const BatchArray& A = arrays[lo];
-    const MaskSpan span = mask_span(A.mask, A.offsets, A.nlists, A.E);
+    const MaskSpan span = mask_span(A.mask, kAnyLength, A.offsets, A.nlists, A.E);
     const long long before = b.tile_before[A.mask_tile0];
     const long long l0 = (g - A.tile0) * kTileLists;
     for (long long l = l0 + threadIdx.x; l < l0 + kTileLists && l < A.nlists; l += kTileBlock) {

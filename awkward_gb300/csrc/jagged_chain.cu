@@ -44,8 +44,9 @@ struct MaskStage {
 
 __global__ void __launch_bounds__(kTileBlock, 6)
     mask_to_index_kernel(int64_t* __restrict__ tooffsets, int64_t* __restrict__ toindex,
-                         const uint8_t* __restrict__ mask, const int64_t* __restrict__ offsets,
-                         long long nlists, long long ntiles, ScanTiles st, uint64_t* err) {
+                         const uint8_t* __restrict__ mask, long long masklen,
+                         const int64_t* __restrict__ offsets, long long nlists, long long ntiles,
+                         ScanTiles st, uint64_t* err) {
   __shared__ TileSmem sm;
   __shared__ MaskTile t;
   __shared__ MaskStage ms;
@@ -53,10 +54,10 @@ __global__ void __launch_bounds__(kTileBlock, 6)
   const long long l0 = tile * kTileLists;
   const long long rem = nlists - l0;
   const int count = (int)(rem < kTileLists ? rem : kTileLists);
-  const long long base = __ldg(offsets + l0);
+  const long long base = end_in_mask(__ldg(offsets + l0), masklen, err);
   for (int i = threadIdx.x; i <= kTileLists; i += kTileBlock) {
     const int k = i < count ? i : count;
-    t.loc[i] = __ldg(offsets + l0 + k) - base;
+    t.loc[i] = end_in_mask(__ldg(offsets + l0 + k), masklen, err) - base;
   }
   if (threadIdx.x == 0) {
     t.base = base;
@@ -206,29 +207,35 @@ template <class W>
 __global__ void __launch_bounds__(kTileBlock, 8)
     mask_select_kernel(int64_t* __restrict__ tooffsets, W* __restrict__ tocontent,
                        int64_t* __restrict__ tocarry, const uint8_t* __restrict__ mask,
-                       const int64_t* __restrict__ offsets, const W* __restrict__ content,
-                       long long nlists, ScanTiles st, uint64_t* err) {
+                       long long masklen, const int64_t* __restrict__ offsets,
+                       const W* __restrict__ content, long long nlists, ScanTiles st,
+                       uint64_t* err) {
   __shared__ MaskSelectSmem sm;
   const long long tile = tile_claim(sm.tile, st);
-  mask_select_tile<W>(sm, tile, nlists, offsets, mask, content, tooffsets, tocontent, tocarry,
-                      nullptr, st, err);
+  mask_select_tile<W>(sm, tile, nlists, offsets, mask, masklen, content, tooffsets, tocontent,
+                      tocarry, nullptr, st, err);
 }
 
 // array[mask] by the bitmap of the whole mask (mask_compact.cuh).
 __global__ void __launch_bounds__(kTileBlock)
-    mask_bits_kernel(MaskBits b, const uint8_t* __restrict__ mask, const int64_t* __restrict__ offsets,
-                     long long nlists, long long nelements) {
+    mask_bits_kernel(MaskBits b, const uint8_t* __restrict__ mask, long long masklen,
+                     const int64_t* __restrict__ offsets, long long nlists, long long nelements,
+                     uint64_t* err) {
   __shared__ MaskBitsSmem sm;
-  mask_bits_tile(sm, b, blockIdx.x, blockIdx.x, mask, mask_span(mask, offsets, nlists, nelements));
+  bool inside;
+  const MaskSpan span = mask_span(mask, masklen, offsets, nlists, nelements, &inside);
+  if (!inside && blockIdx.x == 0 && threadIdx.x == 0) raise_error(err, 0, 0);
+  mask_bits_tile(sm, b, blockIdx.x, blockIdx.x, mask, span);
 }
 
 template <class W, bool CARRY>
 __global__ void __launch_bounds__(kTileBlock, 4)
-    mask_apply_kernel(MaskBits b, const uint8_t* __restrict__ mask, const int64_t* __restrict__ offsets,
-                      long long nlists, long long nelements, const W* __restrict__ content,
+    mask_apply_kernel(MaskBits b, const uint8_t* __restrict__ mask, long long masklen,
+                      const int64_t* __restrict__ offsets, long long nlists, long long nelements,
+                      const W* __restrict__ content,
                       int64_t* __restrict__ tooffsets, W* __restrict__ tocontent,
                       int64_t* __restrict__ tocarry, unsigned copy_blocks) {
-  const MaskSpan span = mask_span(mask, offsets, nlists, nelements);
+  const MaskSpan span = mask_span(mask, masklen, offsets, nlists, nelements);
   if (blockIdx.x < copy_blocks) {
     const long long used = (span.nbits + kChunk - 1) / kChunk;
     const long long step = (long long)copy_blocks * (kTileBlock / 32);
@@ -255,11 +262,12 @@ __global__ void __launch_bounds__(kTileBlock, 4)
 // The new offsets (nlists + 1 entries) and, for each true entry of the mask
 // in order, its position within its list.  toindex must hold as many entries
 // as the mask has true values in the offsets' span (at most offsets[nlists] -
-// offsets[0]).
-GB_EXPORT int awkward_gb300_jagged_mask_to_index(int64_t* tooffsets, int64_t* toindex,
-                                                 const uint8_t* mask, const int64_t* offsets,
-                                                 int64_t nlists, uint64_t* err_code,
-                                                 void* stream) {
+// offsets[0]).  The mask has masklen entries: lists that reach outside them
+// raise code 0 ("index out of range"), and none outside is read.
+GB_EXPORT int awkward_gb300_jagged_mask_to_index_within(int64_t* tooffsets, int64_t* toindex,
+                                                        const uint8_t* mask, int64_t masklen,
+                                                        const int64_t* offsets, int64_t nlists,
+                                                        uint64_t* err_code, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   if (nlists <= 0) return (int)cudaMemsetAsync(tooffsets, 0, sizeof(int64_t), s);
   const long long nt = tile_count(nlists);
@@ -267,11 +275,20 @@ GB_EXPORT int awkward_gb300_jagged_mask_to_index(int64_t* tooffsets, int64_t* to
   void* scratch = nullptr;
   cudaError_t e = scan_tiles_alloc(&st, &scratch, nt, s);
   if (e != cudaSuccess) return (int)e;
-  mask_to_index_kernel<<<(unsigned)nt, kTileBlock, 0, s>>>(tooffsets, toindex, mask, offsets,
-                                                           nlists, nt, st, err_code);
+  mask_to_index_kernel<<<(unsigned)nt, kTileBlock, 0, s>>>(tooffsets, toindex, mask, masklen,
+                                                           offsets, nlists, nt, st, err_code);
   e = cudaGetLastError();
   cudaError_t f = scratch_free(scratch, s);
   return (int)(e != cudaSuccess ? e : f);
+}
+
+// The same with a mask of unknown length, as long as the lists need.
+GB_EXPORT int awkward_gb300_jagged_mask_to_index(int64_t* tooffsets, int64_t* toindex,
+                                                 const uint8_t* mask, const int64_t* offsets,
+                                                 int64_t nlists, uint64_t* err_code,
+                                                 void* stream) {
+  return awkward_gb300_jagged_mask_to_index_within(tooffsets, toindex, mask, kAnyLength, offsets,
+                                                   nlists, err_code, stream);
 }
 
 // out[i] = content[carry[i]] for element widths of 1, 2, 4 and 8 bytes; a carry
@@ -312,11 +329,10 @@ GB_EXPORT int awkward_gb300_take(void* out, const void* content, int64_t itemsiz
 // tocarry is not NULL, each selected element's position in the content (the
 // carry the three-step chain would produce).  tocontent / tocarry hold as many
 // entries as the mask has true values in the offsets' span.
-GB_EXPORT int awkward_gb300_jagged_mask_select(int64_t* tooffsets, void* tocontent,
-                                               int64_t* tocarry, const uint8_t* mask,
-                                               const int64_t* offsets, const void* content,
-                                               int64_t itemsize, int64_t nlists,
-                                               uint64_t* err_code, void* stream) {
+static int mask_select_tiles(int64_t* tooffsets, void* tocontent, int64_t* tocarry,
+                             const uint8_t* mask, int64_t masklen, const int64_t* offsets,
+                             const void* content, int64_t itemsize, int64_t nlists,
+                             uint64_t* err_code, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   if (itemsize != 1 && itemsize != 2 && itemsize != 4 && itemsize != 8)
     return (int)cudaErrorInvalidValue;
@@ -330,41 +346,51 @@ GB_EXPORT int awkward_gb300_jagged_mask_select(int64_t* tooffsets, void* toconte
   switch (itemsize) {
     case 1:
       mask_select_kernel<uint8_t><<<grid, kTileBlock, 0, s>>>(
-          tooffsets, (uint8_t*)tocontent, tocarry, mask, offsets, (const uint8_t*)content,
-          nlists, st, err_code);
+          tooffsets, (uint8_t*)tocontent, tocarry, mask, masklen, offsets,
+          (const uint8_t*)content, nlists, st, err_code);
       break;
     case 2:
       mask_select_kernel<uint16_t><<<grid, kTileBlock, 0, s>>>(
-          tooffsets, (uint16_t*)tocontent, tocarry, mask, offsets, (const uint16_t*)content,
-          nlists, st, err_code);
+          tooffsets, (uint16_t*)tocontent, tocarry, mask, masklen, offsets,
+          (const uint16_t*)content, nlists, st, err_code);
       break;
     case 4:
       mask_select_kernel<uint32_t><<<grid, kTileBlock, 0, s>>>(
-          tooffsets, (uint32_t*)tocontent, tocarry, mask, offsets, (const uint32_t*)content,
-          nlists, st, err_code);
+          tooffsets, (uint32_t*)tocontent, tocarry, mask, masklen, offsets,
+          (const uint32_t*)content, nlists, st, err_code);
       break;
     default:
       mask_select_kernel<uint64_t><<<grid, kTileBlock, 0, s>>>(
-          tooffsets, (uint64_t*)tocontent, tocarry, mask, offsets, (const uint64_t*)content,
-          nlists, st, err_code);
+          tooffsets, (uint64_t*)tocontent, tocarry, mask, masklen, offsets,
+          (const uint64_t*)content, nlists, st, err_code);
   }
   e = cudaGetLastError();
   cudaError_t f = scratch_free(scratch, s);
   return (int)(e != cudaSuccess ? e : f);
 }
 
-// The same with the number of elements in the lists' span, or a bound for it
-// (the mask's length), at hand: where mask_compact() says so the call goes by the
-// bitmap of the whole mask.
-GB_EXPORT int awkward_gb300_jagged_mask_select_sized(int64_t* tooffsets, void* tocontent,
-                                                     int64_t* tocarry, const uint8_t* mask,
-                                                     const int64_t* offsets, const void* content,
-                                                     int64_t itemsize, int64_t nlists,
-                                                     int64_t nelements, uint64_t* err_code,
-                                                     void* stream) {
+GB_EXPORT int awkward_gb300_jagged_mask_select(int64_t* tooffsets, void* tocontent,
+                                               int64_t* tocarry, const uint8_t* mask,
+                                               const int64_t* offsets, const void* content,
+                                               int64_t itemsize, int64_t nlists,
+                                               uint64_t* err_code, void* stream) {
+  return mask_select_tiles(tooffsets, tocontent, tocarry, mask, kAnyLength, offsets, content,
+                           itemsize, nlists, err_code, stream);
+}
+
+// The same with the mask's length and the number of elements in the lists' span,
+// or a bound for it, at hand: where mask_compact() says so the call goes by the
+// bitmap of the whole mask.  Lists that reach outside the mask, or hold more than
+// nelements, raise code 0 ("index out of range"), and no mask entry outside is read.
+GB_EXPORT int awkward_gb300_jagged_mask_select_within(int64_t* tooffsets, void* tocontent,
+                                                      int64_t* tocarry, const uint8_t* mask,
+                                                      int64_t masklen, const int64_t* offsets,
+                                                      const void* content, int64_t itemsize,
+                                                      int64_t nlists, int64_t nelements,
+                                                      uint64_t* err_code, void* stream) {
   if (nlists <= 0 || !mask_compact(nelements, nlists))
-    return awkward_gb300_jagged_mask_select(tooffsets, tocontent, tocarry, mask, offsets, content,
-                                            itemsize, nlists, err_code, stream);
+    return mask_select_tiles(tooffsets, tocontent, tocarry, mask, masklen, offsets, content,
+                             itemsize, nlists, err_code, stream);
   if (itemsize != 1 && itemsize != 2 && itemsize != 4 && itemsize != 8)
     return (int)cudaErrorInvalidValue;
   cudaStream_t s = (cudaStream_t)stream;
@@ -372,13 +398,14 @@ GB_EXPORT int awkward_gb300_jagged_mask_select_sized(int64_t* tooffsets, void* t
   void* tables = nullptr;
   if (scratch_alloc(&tables, mask_bits_bytes(tiles), s) != cudaSuccess) {
     cudaGetLastError();  // no room for the bitmap: the other way needs none
-    return awkward_gb300_jagged_mask_select(tooffsets, tocontent, tocarry, mask, offsets, content,
-                                            itemsize, nlists, err_code, stream);
+    return mask_select_tiles(tooffsets, tocontent, tocarry, mask, masklen, offsets, content,
+                             itemsize, nlists, err_code, stream);
   }
   const MaskBits b = mask_bits_at(tables, tiles);
   cudaError_t e = cudaMemsetAsync(b.finished, 0, sizeof(*b.finished), s);
   if (e == cudaSuccess) {
-    mask_bits_kernel<<<(unsigned)tiles, kTileBlock, 0, s>>>(b, mask, offsets, nlists, nelements);
+    mask_bits_kernel<<<(unsigned)tiles, kTileBlock, 0, s>>>(b, mask, masklen, offsets, nlists,
+                                                            nelements, err_code);
     const long long sms = device_sm_count();
     const long long copies = tiles * (kMaskTile / kChunk) / (kTileBlock / 32);
     const long long lists = (nlists + kTileBlock) / kTileBlock;
@@ -387,8 +414,8 @@ GB_EXPORT int awkward_gb300_jagged_mask_select_sized(int64_t* tooffsets, void* t
 #define GB_MASK_APPLY(W)                                                                       \
   (tocarry ? mask_apply_kernel<W, true> : mask_apply_kernel<W, false>)<<<nc + nl, kTileBlock,  \
                                                                         0, s>>>(               \
-      b, mask, offsets, nlists, nelements, (const W*)content, tooffsets, (W*)tocontent,        \
-      tocarry, nc)
+      b, mask, masklen, offsets, nlists, nelements, (const W*)content, tooffsets,              \
+      (W*)tocontent, tocarry, nc)
     switch (itemsize) {
       case 1: GB_MASK_APPLY(uint8_t); break;
       case 2: GB_MASK_APPLY(uint16_t); break;
@@ -400,4 +427,16 @@ GB_EXPORT int awkward_gb300_jagged_mask_select_sized(int64_t* tooffsets, void* t
   }
   cudaError_t f = scratch_free(tables, s);
   return (int)(e != cudaSuccess ? e : f);
+}
+
+// The same with a mask of unknown length, as long as the lists need.
+GB_EXPORT int awkward_gb300_jagged_mask_select_sized(int64_t* tooffsets, void* tocontent,
+                                                     int64_t* tocarry, const uint8_t* mask,
+                                                     const int64_t* offsets, const void* content,
+                                                     int64_t itemsize, int64_t nlists,
+                                                     int64_t nelements, uint64_t* err_code,
+                                                     void* stream) {
+  return awkward_gb300_jagged_mask_select_within(tooffsets, tocontent, tocarry, mask, kAnyLength,
+                                                 offsets, content, itemsize, nlists, nelements,
+                                                 err_code, stream);
 }

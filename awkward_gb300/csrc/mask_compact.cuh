@@ -70,11 +70,20 @@ struct MaskSpan {
   int shift;
   long long nbits;  // shift + elements of the lists' span (no more than the tables hold)
 };
-__device__ __forceinline__ MaskSpan mask_span(const uint8_t* mask, const int64_t* offsets,
-                                              long long nlists, long long nelements) {
+// The span of lists whose mask has `masklen` entries; *inside is false when it
+// reaches past them or holds more than `nelements`.
+__device__ __forceinline__ MaskSpan mask_span(const uint8_t* mask, long long masklen,
+                                              const int64_t* offsets, long long nlists,
+                                              long long nelements, bool* inside = nullptr) {
   MaskSpan s;
   s.first = __ldg(offsets);
-  long long n = __ldg(offsets + nlists) - s.first;
+  long long last = __ldg(offsets + nlists);
+  if (inside) *inside = s.first >= 0 && last <= masklen && last - s.first <= nelements;
+  if (masklen != kAnyLength) {
+    s.first = s.first < 0 ? 0 : s.first > masklen ? masklen : s.first;
+    last = last > masklen ? masklen : last;
+  }
+  long long n = last - s.first;
   n = n < 0 ? 0 : n > nelements ? nelements : n;
   s.shift = (int)(reinterpret_cast<uintptr_t>(mask + s.first) & 15);
   s.nbits = s.shift + n;

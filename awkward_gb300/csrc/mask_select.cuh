@@ -47,6 +47,15 @@ __device__ __forceinline__ int bitmap_count(const unsigned* bits, int a, int b) 
   return n;
 }
 
+// A list's end inside the mask: an offset below 0 or past its `masklen` entries
+// raises code 0 ("index out of range") and is taken as the nearest inside.
+__device__ __forceinline__ long long end_in_mask(long long o, long long masklen, uint64_t* err) {
+  if (o >= 0 && o <= masklen) return o;
+  raise_error(err, 0, 0);
+  return o < 0 ? 0 : masklen;
+}
+constexpr long long kAnyLength = 0x7fffffffffffffffLL;  // masklen of a mask of unknown length
+
 struct MaskSelectSmem {
   TileSmem tile;
   long long loc[kTileLists + 1];  // list ends relative to the tile's first element
@@ -56,12 +65,14 @@ struct MaskSelectSmem {
 // array[mask] for tile `tile` of the lists offsets[0 .. nlists]: writes the
 // new offsets tooffsets[tile's lists] (and tooffsets[nlists] from the last
 // tile), the selected content, the carry when tocarry is not null and each
-// list's length when tocount is not null.  All threads of the CTA call it.
+// list's length when tocount is not null.  The mask has `masklen` entries
+// (end_in_mask).  All threads of the CTA call it.
 template <class W>
 __device__ __forceinline__ void mask_select_tile(MaskSelectSmem& s, long long tile,
                                                  long long nlists,
                                                  const int64_t* __restrict__ offsets,
                                                  const uint8_t* __restrict__ mask,
+                                                 long long masklen,
                                                  const W* __restrict__ content,
                                                  int64_t* __restrict__ tooffsets,
                                                  W* __restrict__ tocontent,
@@ -71,10 +82,10 @@ __device__ __forceinline__ void mask_select_tile(MaskSelectSmem& s, long long ti
   const long long l0 = tile * kTileLists;
   const long long rem = nlists - l0;
   const int count = (int)(rem < kTileLists ? rem : kTileLists);
-  const long long base = __ldg(offsets + l0);
+  const long long base = end_in_mask(__ldg(offsets + l0), masklen, err);
   for (int i = threadIdx.x; i <= kTileLists; i += kTileBlock) {
     const int k = i < count ? i : count;
-    s.loc[i] = __ldg(offsets + l0 + k) - base;
+    s.loc[i] = end_in_mask(__ldg(offsets + l0 + k), masklen, err) - base;
   }
   __syncthreads();
   const long long total = s.loc[count];

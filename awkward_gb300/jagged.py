@@ -89,6 +89,14 @@ def _array(name, t, dtype=None):
     return t.contiguous()
 
 
+def _mask(mask):
+    """`mask` (bool, or any type of one byte) as contiguous bytes."""
+    m = _array("mask", mask)
+    if m.element_size() != 1:
+        raise TypeError(f"mask must have entries of one byte, not {m.dtype}")
+    return m.view(torch.uint8)
+
+
 def take(content, carry, check=True):
     """content[carry] (a gather); raises ValueError for a carry outside the content."""
     out = torch.empty(carry.numel(), dtype=content.dtype, device=content.device)
@@ -109,15 +117,16 @@ def take(content, carry, check=True):
 
 
 def jagged_mask_to_index(offsets, mask):
-    """(index offsets, local index) of the true entries of a jagged boolean mask."""
+    """(index offsets, local index) of the true entries of a jagged boolean mask;
+    raises ValueError for lists that reach past the mask."""
+    offsets, m = _array("offsets", offsets, torch.int64), _mask(mask)
     n = offsets.numel() - 1
     call = _Call(offsets.device)
-    m = mask.view(torch.uint8) if mask.dtype == torch.bool else mask
     tooffsets = torch.empty(n + 1, dtype=torch.int64, device=offsets.device)
     toindex = torch.empty(max(call.span(offsets, n, m.numel(), 8), 1), dtype=torch.int64,
                           device=offsets.device)
-    rc = _abi.ext_cfunc("awkward_gb300_jagged_mask_to_index")(
-        tooffsets.data_ptr(), toindex.data_ptr(), m.data_ptr(), offsets.data_ptr(), n,
+    rc = _abi.ext_cfunc("awkward_gb300_jagged_mask_to_index_within")(
+        tooffsets.data_ptr(), toindex.data_ptr(), m.data_ptr(), m.numel(), offsets.data_ptr(), n,
         call.address, call.stream)
     if rc != 0:
         raise RuntimeError(f"awkward_gb300_jagged_mask_to_index: cudaError {rc}")
@@ -126,24 +135,26 @@ def jagged_mask_to_index(offsets, mask):
 
 
 def mask_select(offsets, content, mask, with_carry=False):
-    """array[mask] at once (awkward_gb300_jagged_mask_select_sized): the new
+    """array[mask] at once (awkward_gb300_jagged_mask_select_within): the new
     offsets, the selected content and, with `with_carry`, the carry (each
     selected element's position in the content) -- the same outputs as
-    getitem_jagged_mask without its intermediate local index."""
+    getitem_jagged_mask without its intermediate local index.  Raises
+    ValueError for lists that reach past the mask."""
+    offsets, m = _array("offsets", offsets, torch.int64), _mask(mask)
+    content = _array("content", content)
     n = offsets.numel() - 1
     call = _Call(offsets.device)
-    m = mask.view(torch.uint8) if mask.dtype == torch.bool else mask
     itemsize = content.element_size()
     span = max(call.span(offsets, n, m.numel(), itemsize + (8 if with_carry else 0)), 1)
     tooffsets = torch.empty(n + 1, dtype=torch.int64, device=offsets.device)
     out = torch.empty(span, dtype=content.dtype, device=content.device)
     carry = torch.empty(span, dtype=torch.int64, device=offsets.device) if with_carry else None
-    rc = _abi.ext_cfunc("awkward_gb300_jagged_mask_select_sized")(
+    rc = _abi.ext_cfunc("awkward_gb300_jagged_mask_select_within")(
         tooffsets.data_ptr(), out.data_ptr(), carry.data_ptr() if with_carry else None,
-        m.data_ptr(), offsets.data_ptr(), content.data_ptr(), itemsize, n, span,
+        m.data_ptr(), m.numel(), offsets.data_ptr(), content.data_ptr(), itemsize, n, span,
         call.address, call.stream)
     if rc != 0:
-        raise RuntimeError(f"awkward_gb300_jagged_mask_select_sized: cudaError {rc}")
+        raise RuntimeError(f"awkward_gb300_jagged_mask_select_within: cudaError {rc}")
     (k,) = call.finish("awkward_gb300_jagged_mask_select", None, tooffsets.data_ptr() + 8 * n)
     if with_carry:
         return tooffsets, out[:k], carry[:k]

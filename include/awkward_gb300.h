@@ -737,6 +737,9 @@ int awkward_ListArray64_getitem_jagged_apply_64_noalloc(int64_t* tooffsets, int6
  *     (NULL to skip), without the local index of the chain;
  *   jagged_mask_select_sized: the same for a caller who knows the elements in
  *     the lists' span, or no fewer (the mask's length);
+ *   jagged_mask_to_index_within, jagged_mask_select_within: the same for a mask
+ *     of known length -- lists that reach outside its masklen entries set
+ *     err_code to 0 ("index out of range") and none outside is read;
  *   jagged_index_select: array[index] with a jagged int64 index in one pass
  *     -- jagged_apply with the content gathered at each carry (itemsize 1, 2,
  *     4 or 8; tocarry NULL to skip), errors as jagged_apply's;
@@ -751,6 +754,8 @@ int awkward_ListArray64_getitem_jagged_apply_64_noalloc(int64_t* tooffsets, int6
 int awkward_gb300_jagged_mask_to_index(int64_t* tooffsets, int64_t* toindex, const uint8_t* mask, const int64_t* offsets, int64_t nlists, uint64_t* err_code, void* stream);
 int awkward_gb300_jagged_mask_select(int64_t* tooffsets, void* tocontent, int64_t* tocarry, const uint8_t* mask, const int64_t* offsets, const void* content, int64_t itemsize, int64_t nlists, uint64_t* err_code, void* stream);
 int awkward_gb300_jagged_mask_select_sized(int64_t* tooffsets, void* tocontent, int64_t* tocarry, const uint8_t* mask, const int64_t* offsets, const void* content, int64_t itemsize, int64_t nlists, int64_t nelements, uint64_t* err_code, void* stream);
+int awkward_gb300_jagged_mask_to_index_within(int64_t* tooffsets, int64_t* toindex, const uint8_t* mask, int64_t masklen, const int64_t* offsets, int64_t nlists, uint64_t* err_code, void* stream);
+int awkward_gb300_jagged_mask_select_within(int64_t* tooffsets, void* tocontent, int64_t* tocarry, const uint8_t* mask, int64_t masklen, const int64_t* offsets, const void* content, int64_t itemsize, int64_t nlists, int64_t nelements, uint64_t* err_code, void* stream);
 int awkward_gb300_jagged_index_select(int64_t* tooffsets, void* tocontent, int64_t* tocarry, const int64_t* index_offsets, const int64_t* index, int64_t indexlen, const int64_t* offsets, const void* content, int64_t itemsize, int64_t contentlen, int64_t nlists, uint64_t* err_code, void* stream);
 int awkward_gb300_jagged_range_select(int64_t* tooffsets, void* tocontent, int64_t tolen, const int64_t* offsets, const void* content, int64_t itemsize, int64_t contentlen, int64_t nlists, int64_t start, int64_t stop, int64_t step, uint64_t* err_code, void* stream);
 int awkward_gb300_take(void* out, const void* content, int64_t itemsize, const int64_t* carry, int64_t n, int64_t contentlen, uint64_t invocation_index, uint64_t* err_code, void* stream);
