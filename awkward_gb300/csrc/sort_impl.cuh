@@ -52,7 +52,7 @@ static_assert(kSortBlock * kMidItems >= kMidWindow - 1 + kMidMax, "a tile fits i
 // Counter words (device; set to -1 per call, so an add returns one less than
 // the count before it).
 enum { kCntMidTotal = 0, kCntLong = 1, kCntLongTotal = 2, kCntLongMax = 3, kCntLimit = 4,
-       kCntWords = 8 };
+       kCntMerged = 5, kCntWords = 8 };
 static_assert(kCntWords <= Readback::kWords, "the counters are read back in one piece");
 
 // ------------------------------------------------------------ order keys
@@ -312,6 +312,7 @@ struct SortLists {
   long long mid_slots;
   long long* long_st;  // by order of arrival
   long long* long_len;
+  long long* long_base;  // elements before it of segments of several runs
   long long long_cap;
 };
 
@@ -357,6 +358,8 @@ __global__ void __launch_bounds__(kSortBlock, kSmallBlocks)
       if (k < ls.long_cap) {  // beyond it only with overlapping segments
         ls.long_st[k] = st;
         ls.long_len[k] = L;
+        ls.long_base[k] =
+            L > kRun ? (long long)(atomicAdd(ls.counters + kCntMerged, (unsigned long long)L) + 1ull) : 0;
         atomicAdd(ls.counters + kCntLongTotal, (unsigned long long)L);
         atomicMax(reinterpret_cast<long long*>(ls.counters + kCntLongMax), L);
       }
@@ -781,6 +784,7 @@ __device__ __forceinline__ long long warp_find(const long long* __restrict__ fir
 struct LongSegs {
   const long long* st;     // first element
   const long long* len;
+  const long long* base;   // place in the pair buffers, which hold the segments of several runs
   const long long* run0;   // runs of the segments before it
   const long long* total;  // device word: all runs
   long long n;
@@ -789,8 +793,7 @@ struct LongSegs {
 };
 
 // The run of CTA `r` (all threads; false past the last): its segment, first
-// element and the segment's place in the pair buffers, which hold kRun slots
-// per run.
+// element and the segment's place in the pair buffers.
 struct LongRun {
   long long seg, st, len, r0, base;
 };
@@ -806,7 +809,7 @@ __device__ __forceinline__ bool long_run(LongRun& v, const LongSegs& g, long lon
   v.st = g.st[v.seg];
   v.len = g.len[v.seg];
   v.r0 = (r - g.run0[v.seg]) * kRun;
-  v.base = g.run0[v.seg] * kRun;
+  v.base = g.base[v.seg];
   return true;
 }
 
@@ -1071,20 +1074,23 @@ __global__ void __launch_bounds__(kSortBlock)
 
 template <class T, bool ARG, class P>
 cudaError_t sort_long(void* toptr, const T* x, const SortLists& ls, long long nlong, long long total,
-                      long long maxl, bool asc, uint64_t inv, uint64_t* err, cudaStream_t s) {
+                      long long merged, long long maxl, bool asc, uint64_t inv, uint64_t* err,
+                      cudaStream_t s) {
   const long long bound = total / kRun + nlong;  // runs, at most
   const bool merges = maxl > kRun;
-  const size_t pair_bytes = merges ? sizeof(P) * (size_t)bound * kRun : 0;
+  // two pair buffers for the `merged` elements of segments of several runs
+  const size_t pair_bytes = sizeof(P) * (size_t)merged;
   void* mem = nullptr;
   cudaError_t e = scratch_alloc(&mem, 2 * pair_bytes + sizeof(long long) * (size_t)(3 * nlong + 1), s);
   if (e != cudaSuccess) return e;
   P* a = static_cast<P*>(mem);
-  P* b = a + (merges ? bound * kRun : 0);
-  long long* run0 = reinterpret_cast<long long*>(b + (merges ? bound * kRun : 0));
+  P* b = a + merged;
+  long long* run0 = reinterpret_cast<long long*>(b + merged);
   long long* ntotal = run0 + nlong;
   LongSegs g;
   g.st = ls.long_st;
   g.len = ls.long_len;
+  g.base = ls.long_base;
   g.run0 = run0;
   g.total = ntotal;
   g.n = nlong;
@@ -1142,13 +1148,14 @@ cudaError_t launch_sort(void* toptr, const T* x, long long length, const U* offs
   ls.long_cap = length / (kMidMax + 1) + 1 < nseg ? length / (kMidMax + 1) + 1 : nseg;
   void* scratch = nullptr;
   cudaError_t e = scratch_alloc(
-      &scratch, sizeof(long long) * (size_t)(kCntWords + 2 * ls.mid_slots + 2 * ls.long_cap), s);
+      &scratch, sizeof(long long) * (size_t)(kCntWords + 2 * ls.mid_slots + 3 * ls.long_cap), s);
   if (e != cudaSuccess) return e;
   ls.counters = static_cast<unsigned long long*>(scratch);
   ls.mid_st = reinterpret_cast<long long*>(ls.counters + kCntWords);
   ls.mid_len = ls.mid_st + ls.mid_slots;
   ls.long_st = ls.mid_len + ls.mid_slots;
   ls.long_len = ls.long_st + ls.long_cap;
+  ls.long_base = ls.long_len + ls.long_cap;
   e = cudaMemsetAsync(scratch, 0xff, sizeof(long long) * (size_t)(kCntWords + ls.mid_slots), s);
   if (e == cudaSuccess) {
     const long long tiles = (nseg + kSortBlock - 1) / kSortBlock;  // 32 segments a warp
@@ -1176,13 +1183,16 @@ cudaError_t launch_sort(void* toptr, const T* x, long long length, const U* offs
     const long long found = (long long)(rb->words[kCntLong] + 1ull);
     const long long nlong = found < ls.long_cap ? found : ls.long_cap;
     const long long total = (long long)(rb->words[kCntLongTotal] + 1ull);
+    const long long merged = (long long)(rb->words[kCntMerged] + 1ull);
     const long long maxl = (long long)rb->words[kCntLongMax];
     if (e == cudaSuccess && nlong > 0) {
       // a pair's index is 32 bits unless a segment needs more
       if (maxl <= (1ll << 32))
-        e = sort_long<T, ARG, unsigned long long>(toptr, x, ls, nlong, total, maxl, ascending, inv, err, s);
+        e = sort_long<T, ARG, unsigned long long>(toptr, x, ls, nlong, total, merged, maxl, ascending,
+                                                  inv, err, s);
       else
-        e = sort_long<T, ARG, WidePair>(toptr, x, ls, nlong, total, maxl, ascending, inv, err, s);
+        e = sort_long<T, ARG, WidePair>(toptr, x, ls, nlong, total, merged, maxl, ascending, inv,
+                                        err, s);
     }
   }
   cudaError_t f = scratch_free(scratch, s);
