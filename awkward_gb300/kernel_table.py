@@ -32,12 +32,13 @@ from __future__ import annotations
 
 import collections
 import os
+import threading
 
 import numpy as np
 import torch
 
 from . import _abi
-from ._messages import messages
+from ._messages import TIMEOUT_MESSAGE, messages
 from ._signatures import SIGNATURES
 
 ERROR_BITS = 8
@@ -91,13 +92,64 @@ class _Invocation:
         self.keepalive = keepalive
 
 
+class _Pending:
+    """Invocations `first`, `first` + 1, ... of a stream."""
+
+    __slots__ = ("first", "calls")
+
+    def __init__(self, first):
+        self.first = first
+        self.calls = []
+
+    def get(self, number):
+        i = number - self.first
+        return self.calls[i] if 0 <= i < len(self.calls) else None
+
+
 class _StreamContext:
-    """Error word and pending invocations of one stream."""
+    """Error word and pending invocations of one stream, for all threads that use it.
+
+    Invocations are numbered on through every synchronisation, and a number is
+    given out and its kernel launched under the lock.  So whoever takes the
+    pending ones knows that all of them are on the stream, and an error that a
+    later call leaves in the word has a number of its own."""
 
     def __init__(self, device):
         self.err = torch.full((1,), -1, dtype=torch.int64, device=device)  # NO_ERROR
         self.address = self.err.data_ptr()
-        self.pending = []
+        self.lock = threading.Lock()
+        self.pending = _Pending(0)
+        self.taken = []  # by synchronisations that have not read the word yet
+        # (the word of a context made during a capture is filled by the graph's replays)
+        self.captured = torch.cuda.is_current_stream_capturing()
+
+    def launch(self, f, cargs, call, index, stream, fault=None):
+        """f(*cargs, number, word, stream) as the next invocation, and the error
+        code `fault` in its name; f's result."""
+        with self.lock:
+            calls = self.pending.calls
+            number = self.pending.first + len(calls)
+            calls.append(call)
+            rc = f(*cargs, number, self.address, stream)
+            if fault is not None and rc == 0:
+                self.record_error(number, fault, torch.cuda.current_stream(index))
+            return rc
+
+    def take(self):
+        """The pending invocations, for a synchronisation that reads the word next."""
+        with self.lock:
+            p = self.pending
+            self.pending = _Pending(p.first + len(p.calls))
+            self.taken.append(p)
+            return p
+
+    def call(self, number):
+        """The invocation of that number, None when it is no longer known."""
+        for p in (*self.taken, self.pending):
+            c = p.get(number)
+            if c is not None:
+                return c
+        return None
 
     def record_error(self, invocation, code, stream):
         """Lower the error word to invocation*256 + code on `stream` (as atomicMin does)."""
@@ -189,19 +241,13 @@ class GB300Kernel:
             index = torch.cuda.current_device()
         stream = raw_stream(index)
         ctx = self.backend._context(index, stream)
-        if len(ctx.pending) >= MAX_PENDING_INVOCATIONS:
+        if len(ctx.pending.calls) >= MAX_PENDING_INVOCATIONS:
             self.backend.synchronize(torch.cuda.current_stream(index))
             ctx = self.backend._context(index, stream)
-        pending = ctx.pending
-        invocation = len(pending)
-        pending.append(_Invocation(self.family, keep))
-        rc = self._f(*cargs, invocation, ctx.address, stream)
+        fault = injected_fault(self.name, self.family) if FAULT_ENV in os.environ else None
+        rc = ctx.launch(self._f, cargs, _Invocation(self.family, keep), index, stream, fault)
         if rc != 0:
             raise RuntimeError(f"{self.name}: CUDA launch failed with cudaError {rc}")
-        if FAULT_ENV in os.environ:
-            code = injected_fault(self.name, self.family)
-            if code is not None:
-                ctx.record_error(invocation, code, torch.cuda.current_stream(index))
 
 
 class GB300Backend:
@@ -239,7 +285,8 @@ class GB300Backend:
         """The context of raw stream `stream` of device `index`."""
         ctx = self._contexts.get((index, stream))
         if ctx is None:
-            ctx = self._contexts[index, stream] = _StreamContext(torch.device("cuda", index))
+            ctx = self._contexts.setdefault((index, stream),
+                                            _StreamContext(torch.device("cuda", index)))
         return ctx
 
     def selftest_lookback_timeout(self, spin_limit=1000):
@@ -249,11 +296,9 @@ class GB300Backend:
         synchronize() raises the "bounded wait gave up" ValueError."""
         index = torch.cuda.current_device()
         stream = raw_stream(index)
-        ctx = self._context(index, stream)
-        invocation = len(ctx.pending)
-        ctx.pending.append(_Invocation("awkward_gb300_selftest_lookback_timeout", []))
-        rc = _abi.ext_cfunc("awkward_gb300_selftest_lookback_timeout")(
-            int(spin_limit), invocation, ctx.address, stream)
+        name = "awkward_gb300_selftest_lookback_timeout"
+        rc = self._context(index, stream).launch(_abi.ext_cfunc(name), (int(spin_limit),),
+                                                 _Invocation(name, []), index, stream)
         if rc != 0:
             raise RuntimeError(f"look-back self-test: CUDA launch failed with cudaError {rc}")
 
@@ -264,19 +309,34 @@ class GB300Backend:
             stream = current
         index, raw = stream.device.index, stream.cuda_stream
         ctx = self._contexts.get((index, raw))
-        if ctx is None or stream != current:
-            stream.synchronize()
         if ctx is None:
+            stream.synchronize()
             return
-        # reading the word waits for the current stream; without an error the
-        # word is as good as new and the context stays
-        pending, ctx.pending = ctx.pending, []
-        word = int(ctx.err.item()) & NO_ERROR
-        if word == NO_ERROR:
-            return
-        self._contexts[index, raw] = _StreamContext(stream.device)
-        inv = pending[word >> ERROR_BITS]
+        taken = ctx.take()
+        try:
+            # reading the word waits for the current stream; without an error the
+            # word is as good as new and the context stays
+            if stream != current:
+                stream.synchronize()
+            if int(ctx.err.item()) & NO_ERROR == NO_ERROR:
+                return
+            with ctx.lock:  # no launch until the word is clear again
+                stream.synchronize()
+                word = int(ctx.err.item()) & NO_ERROR
+                if word == NO_ERROR:
+                    return  # raised by another thread meanwhile
+                inv = ctx.call(word >> ERROR_BITS)
+                with torch.cuda.stream(stream):
+                    ctx.err.fill_(-1)
+        finally:
+            with ctx.lock:
+                ctx.taken.remove(taken)
+            if ctx.captured:
+                self._contexts.pop((index, raw), None)
         code = word & ((1 << ERROR_BITS) - 1)
+        if inv is None:  # a call that a graph has launched again
+            what = TIMEOUT_MESSAGE if code == TIMEOUT_CODE else f"error {code}"
+            raise ValueError(f"{what} in compiled CUDA code (a replayed call)")
         raise ValueError(f"{messages(inv.name)[code]} in compiled CUDA code ({inv.name})")
 
 

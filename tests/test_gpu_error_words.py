@@ -77,3 +77,88 @@ def test_backend_context_survives_error_free_synchronisations():
     total(out, x, off, 2)
     be.synchronize()
     assert out.tolist() == [3.0, 7.0]
+
+
+def _failing_call(be):
+    import torch
+
+    i8 = torch.empty(4, dtype=torch.int64, device="cuda")
+    off = torch.tensor([0, 3, 5], dtype=torch.int64, device="cuda")
+    return be.by_name("awkward_ListArray64_getitem_jagged_expand_64"), (
+        i8, i8.clone(), torch.zeros(3, dtype=torch.int64, device="cuda"), i8.clone(), off[:-1],
+        off[1:], 2, 2)
+
+
+def test_a_late_error_of_another_thread_has_its_own_name():
+    """A call whose launch is under way when another thread synchronises the same
+    stream: its error is raised once, in its name, by whoever reads it."""
+    import torch
+
+    import awkward_gb300
+
+    be = awkward_gb300.backend()
+    be.synchronize()
+    kernel, args = _failing_call(be)
+    torch.cuda.synchronize()
+    launching, synchronised = threading.Event(), threading.Event()
+    real = kernel._f
+
+    def slow(*cargs):
+        launching.set()
+        synchronised.wait(1.0)
+        return real(*cargs)
+
+    kernel._f = slow
+    raised = []
+    try:
+        other = threading.Thread(target=kernel, args=args)
+        other.start()
+        assert launching.wait(30)
+        for _ in range(2):
+            try:
+                be.synchronize()
+            except ValueError as e:
+                raised.append(str(e))
+            synchronised.set()
+            other.join()
+    finally:
+        kernel._f = real
+    assert len(raised) == 1 and "getitem_jagged_expand" in raised[0]
+    be.synchronize()
+
+
+def test_threads_share_a_stream():
+    import torch
+
+    import awkward_gb300
+
+    be = awkward_gb300.backend()
+    be.synchronize()
+    off = torch.tensor([0, 3, 5], dtype=torch.int64, device="cuda")
+    x = torch.arange(5, dtype=torch.float64, device="cuda")
+    total = be["awkward_reduce_sum", np.float64, np.float64, np.int64]
+    kernel, args = _failing_call(be)
+    torch.cuda.synchronize()
+    errors, others = [], []
+
+    def work(call, n):
+        for _ in range(n):
+            try:
+                call()
+                be.synchronize()
+            except ValueError as e:
+                errors.append(str(e))
+            except BaseException as e:  # noqa: BLE001
+                others.append(repr(e))
+
+    outs = [torch.empty(2, dtype=torch.float64, device="cuda") for _ in range(3)]
+    threads = [threading.Thread(target=work, args=(lambda o=o: total(o, x, off, 2), 300)) for o in outs]
+    threads.append(threading.Thread(target=work, args=(lambda: kernel(*args), 100)))
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    be.synchronize()
+    assert not others
+    assert 0 < len(errors) <= 100 and all("getitem_jagged_expand" in e for e in errors)
+    assert all(o.tolist() == [3.0, 7.0] for o in outs)
