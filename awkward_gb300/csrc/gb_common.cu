@@ -1,6 +1,7 @@
 // gb_common.cu -- host side of the shared infrastructure: the library's
 // stream-ordered scratch pool and cached device properties.
 #include <mutex>
+#include <new>
 
 #include "gb_common.cuh"
 
@@ -52,18 +53,67 @@ cudaError_t scratch_free(void* ptr, cudaStream_t stream) {
   return cudaFreeAsync(ptr, stream);
 }
 
-cudaError_t readback(Readback** out) {
-  static thread_local Readback cache[kMaxDevices];
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+Readback::Buffer* Readback::free_[kMaxDevices] = {};
+
+cudaError_t Readback::take() {
+  cudaError_t e = cudaGetDevice(&device_);
   if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
-  Readback& r = cache[dev];
-  if (!r.words)
-    e = cudaHostAlloc((void**)&r.words, sizeof(unsigned long long) * Readback::kWords, cudaHostAllocDefault);
-  if (e == cudaSuccess && !r.done) e = cudaEventCreateWithFlags(&r.done, cudaEventDisableTiming);
-  *out = &r;
+  if (device_ < 0 || device_ >= kMaxDevices) return cudaErrorInvalidDevice;
+  {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    buffer_ = free_[device_];
+    if (buffer_) free_[device_] = buffer_->next;
+  }
+  if (buffer_) return cudaSuccess;
+  Buffer* b = new (std::nothrow) Buffer;
+  if (!b) return cudaErrorMemoryAllocation;
+  e = cudaHostAlloc((void**)&b->words, sizeof(unsigned long long) * kWords, cudaHostAllocDefault);
+  if (e == cudaSuccess) {
+    e = cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming);
+    if (e != cudaSuccess) cudaFreeHost(b->words);
+  }
+  if (e == cudaSuccess) buffer_ = b;
+  else delete b;
   return e;
+}
+
+cudaError_t Readback::queue(const void* src, int n, cudaStream_t stream) {
+  if (n < 0 || n > kWords - count_) return cudaErrorInvalidValue;
+  cudaError_t e = buffer_ ? cudaSuccess : take();
+  if (e != cudaSuccess) return e;
+  pending_ = true;
+  e = cudaMemcpyAsync(buffer_->words + count_, src, sizeof(unsigned long long) * n,
+                      cudaMemcpyDeviceToHost, stream);
+  count_ += n;
+  if (e != cudaSuccess) buffer_ = nullptr;  // (not used again: see the destructor)
+  return e;
+}
+
+cudaError_t Readback::mark(cudaStream_t stream) {
+  const cudaError_t e = cudaEventRecord(buffer_->done, stream);
+  if (e != cudaSuccess) buffer_ = nullptr;
+  return e;
+}
+
+cudaError_t Readback::wait() {
+  const cudaError_t e = cudaEventSynchronize(buffer_->done);
+  if (e == cudaSuccess) pending_ = false;
+  return e;
+}
+
+cudaError_t Readback::wait_stream(cudaStream_t stream) {
+  const cudaError_t e = cudaStreamSynchronize(stream);
+  if (e == cudaSuccess) pending_ = false;
+  return e;
+}
+
+Readback::~Readback() {
+  // (a buffer that may still be written is not used again: the copy became part
+  // of a graph, or the device has failed)
+  if (!buffer_ || pending_) return;
+  std::lock_guard<std::mutex> lock(g_mutex);
+  buffer_->next = free_[device_];
+  free_[device_] = buffer_;
 }
 
 int device_sm_count() {
@@ -98,13 +148,12 @@ GB_EXPORT int awkward_gb300_read_words(int64_t* dst, const int64_t* const* src, 
                                        void* stream) {
   if (n < 0 || n > gb::Readback::kWords) return (int)cudaErrorInvalidValue;
   cudaStream_t s = (cudaStream_t)stream;
-  gb::Readback* r = nullptr;
-  cudaError_t e = gb::readback(&r);
-  for (int64_t i = 0; i < n && e == cudaSuccess; i++)
-    e = cudaMemcpyAsync(r->words + i, src[i], sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-  cudaError_t w = cudaStreamSynchronize(s);  // also before the buffer is used again
+  gb::Readback r;
+  cudaError_t e = cudaSuccess;
+  for (int64_t i = 0; i < n && e == cudaSuccess; i++) e = r.queue(src[i], 1, s);
+  cudaError_t w = n > 0 ? r.wait_stream(s) : cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = w;
-  for (int64_t i = 0; i < n && e == cudaSuccess; i++) dst[i] = (int64_t)r->words[i];
+  for (int64_t i = 0; i < n && e == cudaSuccess; i++) dst[i] = (int64_t)r.words()[i];
   return (int)e;
 }
 

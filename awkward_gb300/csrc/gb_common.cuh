@@ -39,14 +39,36 @@ cudaError_t scratch_alloc(void** ptr, size_t bytes, cudaStream_t stream);
 cudaError_t scratch_free(void* ptr, cudaStream_t stream);
 // A few device words on their way to the host: a pinned buffer, so that the
 // copies are queued, and an event to wait for them (kernels queued behind it
-// run meanwhile).  One per thread and device; whoever takes it has done with
-// it before it returns.
-struct Readback {
+// run meanwhile).  A call takes one of the device's buffers and gives it back
+// when it returns: there are as many as calls have been under way at once,
+// whatever threads made them.
+class Readback {
+ public:
   static constexpr int kWords = 16;
-  unsigned long long* words = nullptr;
-  cudaEvent_t done = nullptr;
+  // Gives the buffer back, when copies into it can no longer be under way.
+  ~Readback();
+  // Put a copy of the `n` device words at `src` on the stream.
+  cudaError_t queue(const void* src, int n, cudaStream_t stream);
+  // The event that wait() waits for, behind the last copy.
+  cudaError_t mark(cudaStream_t stream);
+  cudaError_t wait();
+  cudaError_t wait_stream(cudaStream_t stream);
+  const unsigned long long* words() const { return buffer_->words; }
+  bool used() const { return buffer_ != nullptr; }
+
+ private:
+  cudaError_t take();
+  struct Buffer {
+    unsigned long long* words = nullptr;
+    cudaEvent_t done = nullptr;
+    Buffer* next = nullptr;
+  };
+  static Buffer* free_[];  // by device
+  Buffer* buffer_ = nullptr;
+  int device_ = 0;
+  int count_ = 0;         // words queued
+  bool pending_ = false;  // copies may be under way
 };
-cudaError_t readback(Readback** out);
 // SM count and the persistent-grid width of the current device (cached).
 int device_sm_count();
 

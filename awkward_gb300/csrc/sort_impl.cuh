@@ -1164,12 +1164,10 @@ cudaError_t launch_sort(void* toptr, const T* x, long long length, const U* offs
         toptr, x, length, offsets, nseg, ascending, ls);
     e = cudaGetLastError();
   }
-  Readback* rb = nullptr;
+  Readback rb;
   if (e == cudaSuccess && length > kMidMax) {
-    e = readback(&rb);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(rb->words, ls.counters, sizeof(long long) * kCntWords, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaEventRecord(rb->done, s);
+    e = rb.queue(ls.counters, kCntWords, s);
+    if (e == cudaSuccess) e = rb.mark(s);
   }
   if (e == cudaSuccess && length > kShortMax) {
     const long long tiles = (length + kMidWindow - 1) / kMidWindow;
@@ -1178,13 +1176,15 @@ cudaError_t launch_sort(void* toptr, const T* x, long long length, const U* offs
         toptr, x, ascending, ls);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess && rb) {
-    e = cudaEventSynchronize(rb->done);
-    const long long found = (long long)(rb->words[kCntLong] + 1ull);
+  if (rb.used()) {  // (whatever failed since: the buffer goes back when its copy is done)
+    const cudaError_t w = rb.wait();
+    if (e == cudaSuccess) e = w;
+    const unsigned long long* words = rb.words();
+    const long long found = (long long)(words[kCntLong] + 1ull);
     const long long nlong = found < ls.long_cap ? found : ls.long_cap;
-    const long long total = (long long)(rb->words[kCntLongTotal] + 1ull);
-    const long long merged = (long long)(rb->words[kCntMerged] + 1ull);
-    const long long maxl = (long long)rb->words[kCntLongMax];
+    const long long total = (long long)(words[kCntLongTotal] + 1ull);
+    const long long merged = (long long)(words[kCntMerged] + 1ull);
+    const long long maxl = (long long)words[kCntLongMax];
     if (e == cudaSuccess && nlong > 0) {
       // a pair's index is 32 bits unless a segment needs more
       if (maxl <= (1ll << 32))
