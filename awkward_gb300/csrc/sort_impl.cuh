@@ -50,9 +50,12 @@ constexpr int kRun = kRunBlock * kRunItems;    // run length of long segments
 static_assert(kSortBlock * kMidItems >= kMidWindow - 1 + kMidMax, "a tile fits its CTA");
 
 // Counter words (device; set to -1 per call, so an add returns one less than
-// the count before it).
+// the count before it).  kCntLong counts the long segments in its low
+// kLongBits bits and, above them, the pairs of those of several runs by
+// sixteens (whole 128-byte lines of pairs).
 enum { kCntMidTotal = 0, kCntLong = 1, kCntLongTotal = 2, kCntLongMax = 3, kCntLimit = 4,
-       kCntMerged = 5, kCntWords = 8 };
+       kCntWords = 8 };
+constexpr int kLongBits = 28;  // (segments of more than kMidMax elements)
 static_assert(kCntWords <= Readback::kWords, "the counters are read back in one piece");
 
 // ------------------------------------------------------------ order keys
@@ -312,7 +315,7 @@ struct SortLists {
   long long mid_slots;
   long long* long_st;  // by order of arrival
   long long* long_len;
-  long long* long_base;  // elements before it of segments of several runs
+  long long* long_base;  // place in the pair buffers (segments of several runs)
   long long long_cap;
 };
 
@@ -354,12 +357,13 @@ __global__ void __launch_bounds__(kSortBlock, kSmallBlocks)
       }
     }
     if (L > kMidMax) {
-      const long long k = (long long)(atomicAdd(ls.counters + kCntLong, 1ull) + 1ull);
+      const unsigned long long pairs = L > kRun ? (unsigned long long)(L + 15) / 16 : 0ull;
+      const unsigned long long before = atomicAdd(ls.counters + kCntLong, pairs << kLongBits | 1ull) + 1ull;
+      const long long k = (long long)(before & ((1ull << kLongBits) - 1ull));
       if (k < ls.long_cap) {  // beyond it only with overlapping segments
         ls.long_st[k] = st;
         ls.long_len[k] = L;
-        ls.long_base[k] =
-            L > kRun ? (long long)(atomicAdd(ls.counters + kCntMerged, (unsigned long long)L) + 1ull) : 0;
+        ls.long_base[k] = (long long)(before >> kLongBits) * 16;
         atomicAdd(ls.counters + kCntLongTotal, (unsigned long long)L);
         atomicMax(reinterpret_cast<long long*>(ls.counters + kCntLongMax), L);
       }
@@ -1180,10 +1184,10 @@ cudaError_t launch_sort(void* toptr, const T* x, long long length, const U* offs
     const cudaError_t w = rb.wait();
     if (e == cudaSuccess) e = w;
     const unsigned long long* words = rb.words();
-    const long long found = (long long)(words[kCntLong] + 1ull);
+    const long long found = (long long)((words[kCntLong] + 1ull) & ((1ull << kLongBits) - 1ull));
     const long long nlong = found < ls.long_cap ? found : ls.long_cap;
     const long long total = (long long)(words[kCntLongTotal] + 1ull);
-    const long long merged = (long long)(words[kCntMerged] + 1ull);
+    const long long merged = (long long)((words[kCntLong] + 1ull) >> kLongBits) * 16;
     const long long maxl = (long long)words[kCntLongMax];
     if (e == cudaSuccess && nlong > 0) {
       // a pair's index is 32 bits unless a segment needs more
