@@ -46,19 +46,18 @@ _LOCAL = threading.local()
 
 
 class _Call:
-    """The stream of one call and the thread's error word there.  Every call
-    reads the word back before it returns and leaves it clear, so the next
-    call of the thread on that stream finds it as a new one."""
+    """The stream of one call and the thread's error word there.  A call takes the
+    word and, when it has read it back and left it clear, puts it by for the next
+    call of the thread on that stream; the word of a call that fails before that
+    (a launch that is refused, a read during a capture) is not used again."""
 
     def __init__(self, device):
-        index = device.index
-        self.stream = raw_stream(index)
-        words = _LOCAL.__dict__.setdefault("words", {})
-        self.err = words.get((index, self.stream))
+        self.key = (device.index, raw_stream(device.index))
+        self.stream = self.key[1]
+        self.words = _LOCAL.__dict__.setdefault("words", {})
+        self.err = self.words.pop(self.key, None)
         if self.err is None:
-            if len(words) >= 64:
-                words.clear()
-            self.err = words[index, self.stream] = torch.full((1,), -1, dtype=torch.int64, device=device)
+            self.err = torch.full((1,), -1, dtype=torch.int64, device=device)
         self.address = self.err.data_ptr()
 
     def finish(self, what, family, *addresses):
@@ -66,6 +65,10 @@ class _Call:
         *got, word = _abi.read_words(self.stream, *addresses, self.address)
         if word != -1:
             self.err.fill_(-1)
+        if len(self.words) >= 64:
+            self.words.clear()
+        self.words[self.key] = self.err
+        if word != -1:
             code = word & 255
             msg = messages(family)[code] if family else (TIMEOUT_MESSAGE if code else "index out of range")
             raise ValueError(f"{msg} in compiled CUDA code ({what})")

@@ -162,3 +162,29 @@ def test_threads_share_a_stream():
     assert not others
     assert 0 < len(errors) <= 100 and all("getitem_jagged_expand" in e for e in errors)
     assert all(o.tolist() == [3.0, 7.0] for o in outs)
+
+
+@pytest.mark.parametrize("failing", ["awkward_gb300_jagged_index_select", "read_words"])
+def test_a_call_that_fails_midway_leaves_no_error_behind(monkeypatch, failing):
+    """The kernel has raised its error, and the call ends before it has read it: by a
+    return code, or by the read itself (as during a capture)."""
+    from awkward_gb300 import _abi
+
+    assert _select(False) == [2.0, 4.0]
+    real_cfunc, real_read = _abi.ext_cfunc, _abi.read_words
+
+    def cfunc(name):
+        f = real_cfunc(name)
+        return (lambda *args: f(*args) or 2) if name == failing else f
+
+    def read(*args):
+        raise RuntimeError("read_words: cudaError 900")
+
+    with monkeypatch.context() as m:
+        m.setattr(_abi, "ext_cfunc", cfunc)
+        if failing == "read_words":
+            m.setattr(_abi, "read_words", read)
+        with pytest.raises(RuntimeError, match="cudaError"):
+            _select(True)
+    assert _select(False) == [2.0, 4.0]
+    _alternate()
