@@ -499,10 +499,8 @@ __device__ __forceinline__ typename Op::Out round_results(const Op& op, TileSpan
   const unsigned lt = (1u << lane) - 1u;
   // the ends, and the lane's K of them; sums read zeros past the span
   if (lane <= K) s.bits[lane] = 0u;
-  if constexpr (W == Walk::kExactSum) {
-    if (n + lane < 32 * K) p[n + lane] = 0.0;
-    if (n + lane + 32 < 32 * K) p[n + lane + 32] = 0.0;
-  }
+  if constexpr (W == Walk::kExactSum)
+    for (int i = n + lane; i < 32 * K; i += 32) p[i] = 0.0;
   __syncwarp();
   const bool some = b > a;
   if (some) atomicOr(s.bits + ((b - 1) >> 5), 1u << ((b - 1) & 31));
