@@ -39,8 +39,11 @@ SLICE_NONE = np.iinfo(np.int64).max  # awkward's kSliceNone
 
 
 # Up to this many bytes a result whose size depends on the data is written into
-# a buffer as long as its source, so that no size is read first.
+# a buffer as long as its source, so that no size is read first -- if the source
+# has no more than _PER_LIST entries a list: a few lists of a large array take a
+# buffer of their own span, after one read of it (about 10 us).
 _WHOLE_SOURCE = 64 << 20
+_PER_LIST = 64
 
 _LOCAL = threading.local()
 
@@ -77,8 +80,10 @@ class _Call:
     def span(self, offsets, n, source, itemsize):
         """Entries to allocate for elements of the lists' span: their number, or
         `source` (no fewer) when that is small enough."""
-        if n <= 0 or source * itemsize <= _WHOLE_SOURCE:
-            return source if n > 0 else 0
+        if n <= 0:
+            return 0
+        if source * itemsize <= _WHOLE_SOURCE and source <= _PER_LIST * n:
+            return source
         first, last = _abi.read_words(self.stream, offsets.data_ptr(), offsets.data_ptr() + 8 * n)
         return last - first
 
@@ -237,8 +242,9 @@ def inner_range(inner_offsets, start=None, stop=None, step=None):
     return nextoffsets, nextcarry[:length]
 
 
-# Up to this many bytes a selection is written into a buffer as long as the
-# content, so that its size need not be counted first.
+# Up to this many bytes a range selection is written into a buffer as long as the
+# content (or the lists' span, when the content has more than _PER_LIST elements a
+# list), so that its size need not be counted first.
 _WHOLE_CONTENT = 1 << 30
 
 
@@ -255,7 +261,15 @@ def range_select(inner_offsets, content, start=None, stop=None, step=None):
     nextoffsets = torch.empty(n + 1, dtype=torch.int64, device=inner_offsets.device)
     size = content.numel()
     call = _Call(content.device)
-    counted = size * content.element_size() > _WHOLE_CONTENT
+    if size > _PER_LIST * n:
+        size = min(size, max(call.span(inner_offsets, n, size, content.element_size()), 0))
+    out = None
+    if size * content.element_size() <= _WHOLE_CONTENT:
+        try:
+            out = torch.empty(max(size, 1), dtype=content.dtype, device=content.device)
+        except torch.cuda.OutOfMemoryError:
+            pass
+    counted = out is None
     if counted:
         be = backend()
         total = torch.empty(1, dtype=torch.int64, device=inner_offsets.device)
@@ -264,7 +278,8 @@ def range_select(inner_offsets, content, start=None, stop=None, step=None):
         be.synchronize()
         size = int(total.item())
     while True:
-        out = torch.empty(max(size, 1), dtype=content.dtype, device=content.device)
+        if out is None:
+            out = torch.empty(max(size, 1), dtype=content.dtype, device=content.device)
         rc = _abi.ext_cfunc("awkward_gb300_jagged_range_select")(
             nextoffsets.data_ptr(), out.data_ptr(), size, inner_offsets.data_ptr(),
             content.data_ptr(), content.element_size(), content.numel(), n, *bounds,
@@ -274,7 +289,8 @@ def range_select(inner_offsets, content, start=None, stop=None, step=None):
         (k,) = call.finish("take", None, nextoffsets.data_ptr() + 8 * n)
         if k <= size:
             break
-        size = k  # overlapping lists: more selected than the content holds
+        # overlapping lists: more selected than the content holds
+        size, out, call = k, None, _Call(content.device)
     # (a small part of the content does not keep a buffer of all of it)
     return nextoffsets, out[:k] if counted or 2 * k >= size else out[:k].clone()
 
