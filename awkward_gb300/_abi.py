@@ -77,10 +77,10 @@ _EXT_CTYPES = {"int64_t": ctypes.c_int64, "uint64_t": ctypes.c_uint64, "int32_t"
 
 def ext_cfunc(name):
     """The typed ctypes function of one extension entry point (_extensions.py)."""
-    from ._extensions import EXTENSIONS
-
     f = _funcs.get(name)
     if f is None:
+        from ._extensions import EXTENSIONS
+
         lib = load_library()
         f = getattr(lib, name)
         args, _group = EXTENSIONS[name]

@@ -94,7 +94,7 @@ def _array(name, t, dtype=None):
         raise TypeError(f"{name} must be a CUDA tensor")
     if dtype is not None and t.dtype is not dtype:
         raise TypeError(f"{name} must have dtype {dtype}, not {t.dtype}")
-    return t.contiguous()
+    return t if t.is_contiguous() else t.contiguous()
 
 
 def _mask(mask):
@@ -102,7 +102,7 @@ def _mask(mask):
     m = _array("mask", mask)
     if m.element_size() != 1:
         raise TypeError(f"mask must have entries of one byte, not {m.dtype}")
-    return m.view(torch.uint8)
+    return m if m.dtype is torch.uint8 else m.view(torch.uint8)
 
 
 def take(content, carry, check=True):
