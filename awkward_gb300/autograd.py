@@ -24,11 +24,12 @@ CUDA kernels; there is no fallback.
 from __future__ import annotations
 
 import math
+import os
 
 import torch
 
 from . import _abi
-from .kernel_table import raw_stream
+from .kernel_table import FAULT_ENV, backend, raw_stream
 
 DEFAULT_ACTIVATION_BUDGET = 256 * 2**20
 
@@ -56,12 +57,15 @@ def _launch(name, *args):
         raise RuntimeError(f"{name}: CUDA launch failed with cudaError {rc}")
 
 
-def _reduce(name, out, values, offsets, *extra):
+def _reduce(name, *args):
     """One of awkward's reducers, straight from the library: it has no error to
     report, and the kernel table would keep the tensors until the next
-    synchronize()."""
-    rc = _abi.cfunc(name)(out.data_ptr(), values.data_ptr(), offsets.data_ptr(), *extra, 0, None,
-                          _stream(values))
+    synchronize().  Through the table where faults are injected."""
+    if FAULT_ENV in os.environ:
+        backend().by_name(name)(*args)
+        return
+    rc = _abi.cfunc(name)(*(a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args),
+                          0, None, _stream(args[0]))
     if rc != 0:
         raise RuntimeError(f"{name}: CUDA launch failed with cudaError {rc}")
 
@@ -97,7 +101,7 @@ class SegmentMax(torch.autograd.Function):
         arg = torch.empty(n, dtype=torch.int64, device=values.device)
         t = _SUFFIX[values.dtype]
         _reduce(f"awkward_reduce_max_{t}_{t}_64", out, values, offsets, n, -math.inf)
-        _reduce(f"awkward_reduce_argmax_{t}_64", arg, values, offsets, offsets.data_ptr(), n)
+        _reduce(f"awkward_reduce_argmax_{t}_64", arg, values, offsets, offsets, n)
         ctx.save_for_backward(arg)
         ctx.nvalues = values.numel()
         return out

@@ -26,6 +26,7 @@ Errors follow awkward's protocol and surface as ``ValueError``.
 
 from __future__ import annotations
 
+import os
 import threading
 
 import numpy as np
@@ -33,7 +34,7 @@ import torch
 
 from . import _abi
 from ._messages import TIMEOUT_MESSAGE, messages
-from .kernel_table import backend, raw_stream
+from .kernel_table import FAULT_ENV, backend, raw_stream
 
 SLICE_NONE = np.iinfo(np.int64).max  # awkward's kSliceNone
 
@@ -297,5 +298,9 @@ def range_select(inner_offsets, content, start=None, stop=None, step=None):
 
 def getitem_inner_range(outer_offsets, inner_offsets, content, start=None, stop=None, step=None):
     """array[..., start:stop:step] of a two-level ListOffsetArray: the outer offsets
-    are unchanged; returns (outer_offsets, new inner offsets, new content)."""
+    are unchanged; returns (outer_offsets, new inner offsets, new content).  By
+    awkward's own steps where faults are injected into them."""
+    if FAULT_ENV in os.environ:
+        nextoffsets, nextcarry = inner_range(inner_offsets, start, stop, step)
+        return outer_offsets, nextoffsets, take(content, nextcarry)
     return (outer_offsets, *range_select(inner_offsets, content, start, stop, step))

@@ -78,3 +78,43 @@ def test_injected_fault_raises_that_code(monkeypatch):
     monkeypatch.delenv(FAULT_ENV)
     k(out, x, off, 3)
     be.synchronize()
+
+
+@pytest.mark.parametrize("kernel", ["awkward_reduce_sum", "awkward_reduce_max", "awkward_reduce_argmax"])
+def test_injected_fault_reaches_the_autograd_reducers(monkeypatch, kernel):
+    import torch
+
+    import awkward_gb300
+    from awkward_gb300 import autograd
+    from awkward_gb300.kernel_table import FAULT_ENV
+
+    be = awkward_gb300.backend()
+    be.synchronize()
+    x = torch.arange(10, dtype=torch.float64, device="cuda", requires_grad=True)
+    off = torch.tensor([0, 3, 3, 10], dtype=torch.int64, device="cuda")
+    monkeypatch.setenv(FAULT_ENV, f"{kernel}:32")
+    total, top = autograd.segment_sum(x, off), autograd.segment_max(x, off)
+    with pytest.raises(ValueError, match=f"bounded wait exceeded.*{kernel}"):
+        be.synchronize()
+    assert total.tolist() == [3.0, 0.0, 42.0] and top.tolist() == [2.0, -np.inf, 9.0]
+    (total.sum() + top[::2].sum()).backward()
+    assert x.grad.tolist() == [1.0, 1.0, 2.0, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, 2.0]
+
+
+@pytest.mark.parametrize("kernel", ["awkward_ListArray_getitem_next_range_carrylength",
+                                    "awkward_ListArray_getitem_next_range"])
+def test_injected_fault_reaches_the_range_slice(monkeypatch, kernel):
+    import torch
+
+    import awkward_gb300
+    from awkward_gb300 import jagged
+    from awkward_gb300.kernel_table import FAULT_ENV
+
+    awkward_gb300.backend().synchronize()
+    x = torch.arange(10, dtype=torch.float64, device="cuda")
+    off = torch.tensor([0, 3, 3, 10], dtype=torch.int64, device="cuda")
+    monkeypatch.setenv(FAULT_ENV, f"{kernel}:32")
+    with pytest.raises(ValueError, match=rf"bounded wait exceeded.*\({kernel}\)"):
+        jagged.getitem_inner_range(off, off, x, 1)
+    monkeypatch.setenv(FAULT_ENV, "awkward_reduce_sum:32")
+    assert jagged.getitem_inner_range(off, off, x, 5)[2].tolist() == [8.0, 9.0]
