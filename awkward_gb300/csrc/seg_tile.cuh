@@ -497,10 +497,11 @@ __device__ __forceinline__ typename Op::Out round_results(const Op& op, TileSpan
   constexpr Walk W = WalkOf<Op>::value;
   constexpr unsigned kFull = 0xffffffffu;
   const unsigned lt = (1u << lane) - 1u;
-  // the ends, and the lane's K of them; sums read zeros past the span
+  // the ends, and the lane's K of them; the lane of the span's end reads zeros past it
+  static_assert(K <= 32);
   if (lane <= K) s.bits[lane] = 0u;
   if constexpr (W == Walk::kExactSum)
-    for (int i = n + lane; i < 32 * K; i += 32) p[i] = 0.0;
+    if (n + lane < 32 * K) p[n + lane] = 0.0;
   __syncwarp();
   const bool some = b > a;
   if (some) atomicOr(s.bits + ((b - 1) >> 5), 1u << ((b - 1) & 31));
@@ -530,17 +531,21 @@ __device__ __forceinline__ typename Op::Out round_results(const Op& op, TileSpan
       bad = 0;
       w = Wide{0, 0};
       unsigned r = (unsigned)__cvta_generic_to_shared(s.r.sums + r0);
+      if (q0 < n) {
 #pragma unroll
-      for (int k = 0; k < K; k++) {
-        wide_add(w, q[k], state.low, bad);
-        push_if(ends & 1u << k, r, w);
+        for (int k = 0; k < K; k++) {
+          wide_add(w, q[k], state.low, bad);
+          push_if(ends & 1u << k, r, w);
+        }
       }
       if (!__any_sync(kFull, bad != 0u) || attempt == 1) break;
       unsigned top = 0;  // the window below this round's largest element, one binade to spare
+      if (q0 < n) {
 #pragma unroll
-      for (int k = 0; k < K; k++) {
-        const unsigned u = 2u * (unsigned)__double2hiint(q[k]);
-        top = u > top ? u : top;
+        for (int k = 0; k < K; k++) {
+          const unsigned u = 2u * (unsigned)__double2hiint(q[k]);
+          top = u > top ? u : top;
+        }
       }
       if (!move_window(state.low, top)) break;
     }

@@ -299,8 +299,9 @@ def range_select(inner_offsets, content, start=None, stop=None, step=None):
 def getitem_inner_range(outer_offsets, inner_offsets, content, start=None, stop=None, step=None):
     """array[..., start:stop:step] of a two-level ListOffsetArray: the outer offsets
     are unchanged; returns (outer_offsets, new inner offsets, new content).  By
-    awkward's own steps where faults are injected into them."""
-    if FAULT_ENV in os.environ:
+    awkward's own steps where faults are injected into them, and for wider items
+    than the library gathers (an empty selection of them needs no gather)."""
+    if FAULT_ENV in os.environ or content.element_size() > 8:
         nextoffsets, nextcarry = inner_range(inner_offsets, start, stop, step)
         return outer_offsets, nextoffsets, take(content, nextcarry)
     return (outer_offsets, *range_select(inner_offsets, content, start, stop, step))

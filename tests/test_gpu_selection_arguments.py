@@ -116,3 +116,18 @@ def test_nothing_is_written_past_a_short_masks_result(n, lists):
         to.data_ptr(), index.data_ptr(), m.data_ptr(), short, off.data_ptr(), lists,
         err.data_ptr(), stream) == 0
     assert err.item() == 0 and int(to[-1]) == short and bool((index[short:] == -7).all())
+
+
+@pytest.mark.gpu
+def test_range_of_wide_items():
+    """Items of 16 bytes are not gathered; a selection without any needs no gather."""
+    import torch
+
+    from awkward_gb300 import jagged
+
+    off = torch.tensor([0, 3, 3, 5], dtype=torch.int64, device="cuda")
+    x = torch.zeros(5, dtype=torch.complex128, device="cuda")
+    _, nextoffsets, out = jagged.getitem_inner_range(off, off, x, 3)
+    assert nextoffsets.tolist() == [0, 0, 0, 0] and out.numel() == 0 and out.dtype == x.dtype
+    with pytest.raises(RuntimeError, match="cudaError 1$"):
+        jagged.getitem_inner_range(off, off, x, 1)
