@@ -314,6 +314,12 @@ struct WalkState<ExtremumOp<T, MAX>> {
   const T* x;
 };
 
+template <class T, bool MAX>
+__device__ __forceinline__ tile_key_t<T> ident_key(const ExtremumOp<T, MAX>& op) {
+  using Key = tile_key_t<T>;
+  return is_nan(op.ident) ? (Key)~((Key)1 << (8 * sizeof(Key) - 1)) : tile_key<T, MAX>(op.ident);
+}
+
 // The window below the largest element `top` of a round (hi words doubled, all
 // lanes'), one binade to spare; false when there is none.
 __device__ __forceinline__ bool move_window(unsigned& low, unsigned top) {
@@ -402,7 +408,7 @@ __device__ __forceinline__ typename Op::Out lane_results(const Op& op,
 // other: `p` is the span in shared memory, the lane's list its n elements from a
 // on, `lists` of them.
 template <class Op>
-__device__ __forceinline__ typename Op::Out warp_results(const Op& op,
+__device__ __forceinline__ typename Op::Out warp_each_results(const Op& op,
                                                          const store_t<typename Op::In>* p, int lists,
                                                          int n, int a, int lane, WalkState<Op>& state,
                                                          bool& done) {
@@ -482,6 +488,157 @@ __device__ __forceinline__ typename Op::Out warp_results(const Op& op,
     if (lane == l) mine = v;
   }
   return mine;
+}
+
+// The same for the extrema of 4-byte elements: two or four lists at once, with 16 or 8
+// lanes on each (float32 lists of mean 100 to 220, 16M elements: max 34-42 -> 30-34 us;
+// the others' kernels have no registers left for it).
+template <class Op>
+__device__ __forceinline__ typename Op::Out group_results(const Op& op,
+                                                          const store_t<typename Op::In>* p, int lists,
+                                                          int n, int a, int lane,
+                                                          const WalkState<Op>& state) {
+  using T = store_t<typename Op::In>;
+  constexpr unsigned kFull = 0xffffffffu;
+  typename Op::Out mine{};
+  constexpr bool MAX = WalkOf<Op>::kMax;
+  using Key = tile_key_t<T>;
+  const int lanes = lists > 2 ? 8 : lists > 1 ? 16 : 32;
+  const int group = lane / lanes, sub = lane & (lanes - 1);
+  for (int l = 0; l < lists; l += 32 / lanes) {
+    const int few = lists - l < 32 / lanes ? lists - l : 32 / lanes;
+    const int of = l + (group < few ? group : 0);  // the lane's list
+    const int first = __shfl_sync(kFull, a, of);
+    const int m = __shfl_sync(kFull, n, of);
+    const T* q = p + first;
+    // (a lane past the end takes the last element)
+    Key best = tile_key<T, MAX>(q[sub < m ? sub : m - 1]);
+    for (int i = sub + lanes; i < m; i += lanes) {
+      const Key k = tile_key<T, MAX>(q[i]);
+      best = k > best ? k : best;
+    }
+    for (int d = lanes >> 1; d > 0; d >>= 1) {
+      const Key o = __shfl_xor_sync(kFull, best, d);
+      best = o > best ? o : best;
+    }
+    const T x = tile_value<T, MAX>(best);
+    const bool exact = winner_exact(x);
+    typename Op::Out v = best > state.ident ? x : op.ident;
+    // a zero or a NaN won: the exact rules, by the whole warp
+    for (unsigned rest = __ballot_sync(kFull, !exact); rest;) {
+      const int from = __ffs(rest) - 1;
+      const int f = __shfl_sync(kFull, first, from), c = __shfl_sync(kFull, m, from);
+      typename Op::Acc acc = op.identity();
+      for (int i = lane; i < c; i += 32) acc = op.step(acc, p[f + i], f + i, i == 0, 0);
+      const typename Op::Out w = op.finalize(warp_allreduce(op, acc), 0);
+      if (first == f) v = w;
+      rest &= ~__ballot_sync(kFull, first == f);
+    }
+    const typename Op::Out w = __shfl_sync(kFull, v, (lane - l) * lanes & 31);
+    if (lane >= l && lane < l + few) mine = w;
+  }
+  return mine;
+}
+template <class Op>
+__device__ __forceinline__ typename Op::Out warp_results(const Op& op,
+                                                         const store_t<typename Op::In>* p, int lists,
+                                                         int n, int a, int lane, WalkState<Op>& state,
+                                                         bool& done) {
+  if constexpr (WalkOf<Op>::value == Walk::kExtremum && sizeof(store_t<typename Op::In>) == 4)
+    return group_results(op, p, lists, n, a, lane, state);
+  else
+    return warp_each_results(op, p, lists, n, a, lane, state, done);
+}
+
+// A range whose lists of 8-byte elements have a mean of kWarpList and more, and none
+// of which is longer than a round holds, is taken 32 lists at a time without a copy:
+// a round would hold one to three of them.  Four at once, eight lanes on each, straight
+// from memory.  16M elements in lists of mean 100, 150 and 220: argmax of doubles 57,
+// 57, 47 -> 46, 43, 44 us, max of int64 49, 48, 40 -> 41, 40, 42, argmax 50, 50, 41 ->
+// 43, 41, 42.  The sums and the maxima of doubles stay with the rounds: their kernels
+// have no registers left, and every length paid for it (max at mean 8 44 -> 53 us; sums
+// of lists of 290 to 400 51 -> 62, of mean 100 73 -> 58).
+template <class Op>
+constexpr bool kDirect =
+    sizeof(store_t<typename Op::In>) == 8 &&
+    (WalkOf<Op>::value == Walk::kArg ||
+     (WalkOf<Op>::value == Walk::kExtremum && std::is_integral<typename Op::In>::value));
+
+// The results of such lists: x is the first one's first element, the lane's list its n
+// elements from a on, `lists` of them.
+template <class Op>
+__device__ __forceinline__ typename Op::Out direct_results(const Op& op,
+                                                           const store_t<typename Op::In>* x, int lists,
+                                                           int n, int a, int lane,
+                                                           const WalkState<Op>& state) {
+  using T = store_t<typename Op::In>;
+  using Out = typename Op::Out;
+  constexpr Walk W = WalkOf<Op>::value;
+  constexpr unsigned kFull = 0xffffffffu;
+  constexpr int kFlight = 8;
+  const int sub = lane & 7;
+  tile_key_t<T> top = 0;  // of the lane's list: its winner
+  int place = 0;
+  for (int l = 0; l < lists; l += 4) {
+    const int of = l + (lane >> 3);
+    const T* q = x + __shfl_sync(kFull, a, of & 31);
+    int m = __shfl_sync(kFull, n, of & 31);
+    if (of >= lists) m = 0;
+    const int longest = __reduce_max_sync(kFull, m);
+    const int from = (lane - l) * 8 & 31;  // the lane with its list's result, if it is one of the four
+    const bool mine = lane >= l && lane < l + 4;
+    constexpr bool MAX = WalkOf<Op>::kMax;
+    using Key = tile_key_t<T>;
+    constexpr Key kLowest = (Key)((unsigned long long)1 << (8 * sizeof(Key) - 1));
+    Key best = kLowest;
+    int at = 0x7fffffff;  // (none)
+    for (int i = sub; i < longest; i += 8 * kFlight) {
+      T v[kFlight];
+#pragma unroll
+      for (int u = 0; u < kFlight; u++) v[u] = i + 8 * u < m ? __ldg(q + i + 8 * u) : T(0);
+#pragma unroll
+      for (int u = 0; u < kFlight; u++) {
+        const Key k = tile_key<T, MAX>(v[u]);
+        const bool take = i + 8 * u < m && (k > best || at == 0x7fffffff);
+        best = take ? k : best;
+        at = take ? i + 8 * u : at;
+      }
+    }
+#pragma unroll
+    for (int d = 4; d > 0; d >>= 1) {
+      const Key o = __shfl_xor_sync(kFull, best, d);
+      const int oa = __shfl_xor_sync(kFull, at, d);
+      if (o > best || (o == best && oa < at)) {
+        best = o;
+        at = oa;
+      }
+    }
+    best = __shfl_sync(kFull, best, from);
+    at = __shfl_sync(kFull, at, from);
+    if (mine) {
+      top = best;
+      place = at;
+    }
+  }
+  const T winner = tile_value<T, WalkOf<Op>::kMax>(top);
+  bool exact = n <= 0 || winner_exact(winner);
+  Out v;
+  if constexpr (W == Walk::kArg) {
+    if (std::is_floating_point<T>::value) exact = exact && !(n > 0 && is_nan(__ldg(x + a)));
+    v = n > 0 ? a + place : -1;
+  } else {
+    v = n > 0 && top > state.ident ? winner : op.ident;
+  }
+  // a zero or a NaN won: the exact rules, by the whole warp
+  for (unsigned rest = __ballot_sync(kFull, !exact); rest; rest &= rest - 1) {
+    const int of = __ffs(rest) - 1;
+    const int first = __shfl_sync(kFull, a, of), m = __shfl_sync(kFull, n, of);
+    typename Op::Acc acc = op.identity();
+    for (int i = lane; i < m; i += 32) acc = op.step(acc, __ldg(x + first + i), first + i, i == 0, 0);
+    const Out w = op.finalize(warp_allreduce(op, acc), 0);
+    if (lane == of) v = w;
+  }
+  return v;
 }
 
 // The results of a round's lists, element-parallel: `p` is the span in shared
@@ -840,6 +997,30 @@ __device__ __forceinline__ void seg_tile_range(const Op& op,
     l = l < lists ? l : lists - 1;
     return __ldg(ends + 2 * (long long)l);  // (nothing waits for it here)
   };
+  if constexpr (kDirect<Op>) {
+    const int n = (int)((unsigned)__ldg(ends + 2 * (long long)(lists - 1)) - (unsigned)first);
+    bool direct = n >= (long long)lists * kWarpList;
+    for (int b = 0; b < lists && direct; b += 32) {
+      const int en = load_end(b + lane), up = __shfl_up_sync(kFull, en, 1);
+      const int st = lane ? up : b ? load_end(b - 1) : first;
+      direct = __all_sync(kFull, (unsigned)en - (unsigned)st <= (unsigned)kSpan<T>);
+    }
+    if (direct) {
+      WalkState<Op> state;
+      if constexpr (WalkOf<Op>::value == Walk::kExtremum) state.ident = ident_key(op);
+      for (int b = 0; b < lists; b += 32) {
+        const int c = lists - b < 32 ? lists - b : 32;
+        const int en = load_end(b + lane), up = __shfl_up_sync(kFull, en, 1);
+        const int st = lane ? up : b ? load_end(b - 1) : first;
+        const int at = (int)((unsigned)st - (unsigned)first);
+        typename Op::Out v = direct_results(op, xr, c, lane < c ? (int)((unsigned)en - (unsigned)st) : 0,
+                                            at, lane, state);
+        if constexpr (WalkOf<Op>::value == Walk::kArg) v = v < 0 ? v : v + lo;
+        if (lane < c) to[b + lane] = v;
+      }
+      return;
+    }
+  }
   // the round from list b, element l on, with the lanes' loaded ends: its
   // lists (0 when the first is too long for one), their ends relative to l,
   // its elements and where it ends
@@ -860,9 +1041,7 @@ __device__ __forceinline__ void seg_tile_range(const Op& op,
   };
   WalkState<Op> state;
   if constexpr (WalkOf<Op>::value == Walk::kExtremum) {
-    using Key = tile_key_t<T>;
-    state.ident = is_nan(op.ident) ? (Key)~((Key)1 << (8 * sizeof(Key) - 1))
-                                   : tile_key<T, WalkOf<Op>::kMax>(op.ident);
+    state.ident = ident_key(op);
     state.x = xr;
   }
   // list ends are loaded two rounds ahead, elements copied one ahead
