@@ -177,9 +177,9 @@ __global__ void __launch_bounds__(kSortBlock)
 // top bits of a floating-point key; otherwise the keys less the segment's
 // smallest, shifted to fit), and the network is as wide as the warp's longest
 // segment needs (Batcher's for 8, 16, 24 or 32).  A segment with neighbours
-// that tie in the kept bits while others were dropped is finished by insertion
-// by its whole keys, after a second try when many have some (short_order).  The
-// order goes back through the stage, for coalesced stores.
+// that tie in the kept bits while others were dropped is finished by an
+// insertion sort on its whole keys.  The order goes back through the stage,
+// for coalesced stores.
 //
 // Bound by instructions (ALU 73 %; DRAM traffic is the input and output once).
 // argsort of 2M float64 lists of mean 8: 80 us, against 166 us for counting
@@ -193,22 +193,19 @@ __global__ void __launch_bounds__(kSortBlock)
 constexpr int kShortStage = 4096;  // bytes of a warp's stage: 16 segments always fit
 constexpr int kSmallBlocks = 4;    // resident CTAs per SM (32 registers hold the widest network)
 constexpr int kListStep = kShortMax + 1;
-// Lanes of a warp with ties from which its 32 floating-point segments are staged again
-// by the range of their own keys.  2M float64 lists of mean 8 whose values are within
-// 2^-20 of each other: CLOSER_FIGURES.
-constexpr int kCloserLanes = 8;
-constexpr int kCloserBits = 4;
 
 // The staged word of a value: its order key, for double the high word of it.
 template <class T>
 using stage_t = typename std::conditional<std::is_same<T, double>::value, unsigned, okey_t<T>>::type;
+// (A double's is never above a larger double's: the values next to the zeros
+// with a negative sign share the zeros' word, and are told apart as ties.)
 template <class T>
 __device__ __forceinline__ stage_t<T> stage_word(T v, bool asc) {
   if constexpr (std::is_same<T, double>::value) {
     const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
     const unsigned mag = hi & 0x7fffffffu;
     unsigned k = hi ^ ((unsigned)((int)hi >> 31) | 0x80000000u);
-    if (hi == 0x80000000u && lo == 0u) k = hi;
+    if (hi == 0x80000000u) k = hi;
     k = asc ? k : ~k;
     return mag > 0x7ff00000u || (mag == 0x7ff00000u && lo != 0u) ? 0u : k;  // NaN first
   } else {
@@ -236,34 +233,16 @@ __device__ __forceinline__ void sort_network(unsigned (&c)[N]) {
   }
 }
 
-// What a stage of floating-point words holds: the keys' upper bits, or (closer) the
-// keys less the smallest of the stage, aligned to their largest difference.
-template <class T>
-struct StageRange {
-  okey_t<T> lo = 0;
-  int width = 8 * (int)sizeof(T);  // bits of the largest difference
-  bool closer = false;
-  __device__ __forceinline__ unsigned word(T v, bool asc) const {
-    const okey_t<T> d = order_key<T>(v, asc) - lo;
-    return width > 32 ? (unsigned)((unsigned long long)d >> (width - 32))
-                      : width > 0 ? (unsigned)d << (32 - width) : 0u;
-  }
-};
-
 // The lane's segment (n <= N staged words from slot loc; its values at xs):
 // leaves its order in the stage as 32-bit words, position + `base`.  Whole warp.
-// False, and the stage as it was, when kCloserLanes lanes and more have neighbours
-// that tie and the stage holds the keys' upper bits.
 template <int N, class T>
-__device__ __forceinline__ bool short_order(unsigned char* stage, int loc, int n,
-                                            const T* __restrict__ xs, bool asc, int base,
-                                            const StageRange<T>& range) {
+__device__ __forceinline__ void short_order(unsigned char* stage, int loc, int n,
+                                            const T* __restrict__ xs, bool asc, int base) {
   using W = stage_t<T>;
   const W* word = reinterpret_cast<const W*>(stage) + loc;
   unsigned c[N];
   bool dropped = true;
   if constexpr (std::is_floating_point<T>::value) {
-    dropped = range.width > 27;
 #pragma unroll
     for (int j = 0; j < N; j++) {
       c[j] = ~0u;
@@ -304,36 +283,29 @@ __device__ __forceinline__ bool short_order(unsigned char* stage, int loc, int n
     }
   }
   sort_network(c);
-  bool tie = false;
-#pragma unroll
-  for (int j = 1; j < N; j++) tie |= (c[j] ^ c[j - 1]) < 32u && j < n;
-  tie = tie && dropped;
-  if constexpr (std::is_floating_point<T>::value)
-    if (!range.closer && __popc(__ballot_sync(0xffffffffu, tie)) >= kCloserLanes) return false;
   __syncwarp();  // every lane has read its words
   unsigned* order = reinterpret_cast<unsigned*>(stage) + loc;
+  bool tie = false;
 #pragma unroll
-  for (int j = 0; j < N; j++)
-    if (j < n) order[j] = tie ? c[j] : (c[j] & 31u) + base;
-  if (tie) {  // each run of ties by insertion
+  for (int j = 0; j < N; j++) {
+    if (j < n) order[j] = (c[j] & 31u) + base;
+    if (j > 0) tie |= (c[j] ^ c[j - 1]) < 32u && j < n;
+  }
+  if (tie && dropped) {
     for (int j = 1; j < n; j++) {
       const unsigned e = order[j];
-      if ((e ^ order[j - 1]) >= 32u) continue;
-      const okey_t<T> k = order_key<T>(xs[e & 31u], asc);
+      const okey_t<T> k = order_key<T>(xs[e - base], asc);
       int i = j;
       for (; i > 0; i--) {
         const unsigned o = order[i - 1];
-        if ((e ^ o) >= 32u) break;
-        const okey_t<T> ko = order_key<T>(xs[o & 31u], asc);
-        if (ko < k || (ko == k && (o & 31u) < (e & 31u))) break;
+        const okey_t<T> ko = order_key<T>(xs[o - base], asc);
+        if (ko < k || (ko == k && o < e)) break;
         order[i] = o;
       }
       order[i] = e;
     }
-    for (int j = 0; j < n; j++) order[j] = (order[j] & 31u) + base;
   }
   __syncwarp();
-  return true;
 }
 
 struct SortLists {
@@ -443,40 +415,10 @@ __global__ void __launch_bounds__(kSortBlock, kSmallBlocks)
       // (a sort's order holds places in the stage while the segments are
       // contiguous there and in memory: the values follow without a look-up)
       const int base = !ARG && chain ? loc : 0;
-      StageRange<T> range;
-#pragma unroll 1
-      while (true) {
-        bool done;
-        if (longest <= 8) done = short_order<8>(s_stage[w], loc, mine, x + st, asc, base, range);
-        else if (longest <= 16) done = short_order<16>(s_stage[w], loc, mine, x + st, asc, base, range);
-        else if (longest <= 24) done = short_order<24>(s_stage[w], loc, mine, x + st, asc, base, range);
-        else done = short_order<32>(s_stage[w], loc, mine, x + st, asc, base, range);
-        if (done) break;
-        // the stage's own range: its words again by it where it gains kCloserBits
-        range.closer = true;
-        if (!chain) continue;
-        okey_t<T> lo = ~okey_t<T>(0), hi = 0;
-#pragma unroll 4
-        for (int e = lane; e < cnt; e += 32) {
-          const okey_t<T> k = order_key<T>(x[st0 + e], asc);
-          lo = k < lo ? k : lo;
-          hi = k > hi ? k : hi;
-        }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-          const okey_t<T> a = __shfl_xor_sync(0xffffffffu, lo, d), b = __shfl_xor_sync(0xffffffffu, hi, d);
-          lo = a < lo ? a : lo;
-          hi = b > hi ? b : hi;
-        }
-        const int width = 64 - __clzll((long long)(hi - lo));
-        if (width + kCloserBits > (int)(8 * sizeof(T))) continue;
-        range.lo = lo;
-        range.width = width;
-        if (width > 0)  // (else every key is the same: positions decide)
-#pragma unroll 4
-          for (int e = lane; e < cnt; e += 32) word[e] = range.word(x[st0 + e], asc);
-        __syncwarp();
-      }
+      if (longest <= 8) short_order<8>(s_stage[w], loc, mine, x + st, asc, base);
+      else if (longest <= 16) short_order<16>(s_stage[w], loc, mine, x + st, asc, base);
+      else if (longest <= 24) short_order<24>(s_stage[w], loc, mine, x + st, asc, base);
+      else short_order<32>(s_stage[w], loc, mine, x + st, asc, base);
       if (chain) {
 #pragma unroll 4
         for (int e = lane; e < cnt; e += 32) {
@@ -692,49 +634,6 @@ __device__ __forceinline__ bool fix_ties(Tile& s, int count, Full full, Lo seg_l
   return true;
 }
 
-// When that fails: the runs of ties numbered in order, and the slots sorted by that
-// number and the next of the `left` dropped bits, as many as fit 32 bits with it.
-// dropped(idx) are a slot's dropped bits.  Returns the bits still not looked at (0:
-// slots with equal keys have equal full keys).
-//
-// A second sort of the dropped bits and then the kept ones again took twice the
-// passes: TIES_FIGURES.
-template <class Tile, class Dropped, class Lo>
-__device__ __forceinline__ int split_ties(Tile& s, int count, int nitems, int left, Dropped dropped,
-                                          Lo seg_lo) {
-  constexpr int THREADS = Tile::kThreads, ITEMS = Tile::kItems;
-  __syncthreads();
-  const int q0 = threadIdx.x * ITEMS;
-  unsigned first = 0, begins = 0;  // a bit per slot of the thread: a run begins there
-#pragma unroll
-  for (int j = 0; j < ITEMS; j++) {
-    const int q = q0 + j;
-    if (q < count && (q == seg_lo(q) || s.key[q] != s.key[q - 1])) begins |= 1u << j;
-  }
-  unsigned total;
-  auto add = [](unsigned a, unsigned b) { return a + b; };
-  first = block_exclusive_scan<THREADS>((unsigned)__popc(begins), add, 0u, s.scan, &total);
-  const int bits = total > 1 ? 32 - __clz((int)(total - 1)) : 0;
-  const int take = left < 32 - bits ? left : 32 - bits;
-  left -= take;
-  const unsigned long long mask = (1ull << take) - 1ull;
-  __syncthreads();  // (every key has been compared)
-#pragma unroll
-  for (int j = 0; j < ITEMS; j++) {
-    const int q = q0 + j;
-    if (q >= nitems * THREADS) break;
-    unsigned k = ~0u;
-    if (q < count) {
-      const unsigned run = first + __popc(begins & ((2u << j) - 1u)) - 1u;
-      k = (unsigned)((unsigned long long)run << take | (dropped(s.idx[q]) >> left & mask));
-    }
-    s.key[q] = k;
-  }
-  __syncthreads();
-  radix_bits<Tile>(nitems, bits + take);
-  return left;
-}
-
 // ------------------------------------------------------------ tiles of whole segments
 // The listed segments of kShortMax+1 .. kMidMax elements.  A tile is the
 // segments whose base (the elements listed before them) lies in a window of
@@ -833,10 +732,23 @@ __global__ void __launch_bounds__(kSortBlock, 4)
     if constexpr (sizeof(T) > 4) {
       auto seg_lo = [&](int q) { return s_loc[s_of[q]]; };
       auto seg_hi = [&](int q) { return s_loc[s_of[q] + 1]; };
-      auto whole = [&](int i) { return (unsigned long long)full(i); };
-      auto dropped = [&](int i) { return (unsigned long long)(full(i) - lo); };
-      for (int left = shift; left > 0 && !fix_ties(s, count, whole, seg_lo, seg_hi);)
-        left = split_ties(s, count, nitems, left, dropped, seg_lo);
+      if (shift > 0 && !fix_ties(s, count, [&](int i) { return (unsigned long long)full(i); }, seg_lo,
+                                 seg_hi)) {
+        // many ties of different keys: all the bits, the dropped ones first
+        for (int q = threadIdx.x; q < nitems * kSortBlock; q += kSortBlock) {
+          s.key[q] = q < count ? (unsigned)((full(q) - lo) & ((1ull << shift) - 1ull)) : ~0u;
+          s.idx[q] = (unsigned short)q;
+        }
+        __syncthreads();
+        radix_bits<Tile>(nitems, shift);
+        for (int q = threadIdx.x; q < nitems * kSortBlock; q += kSortBlock) {
+          const int i = s.idx[q];
+          s.key[q] = i < count ? (unsigned)((full(i) - lo) >> shift) : ~0u;
+        }
+        __syncthreads();
+        radix_bits<Tile>(nitems, width - shift);
+        if (nseg > 1) radix_pass<Tile>(nitems, -1);
+      }
     }
     for (int q = threadIdx.x; q < count; q += kSortBlock) {
       const int g = s_of[q], b = s_loc[g];
@@ -1001,16 +913,19 @@ __global__ void __launch_bounds__(kRunBlock)
   radix_bits<Tile>(nitems, width - shift);
   if constexpr (sizeof(T) > 4) {
     auto full = [&](int i) { return (unsigned long long)order_key<T>(xr[i], asc); };
-    auto dropped = [&](int i) { return full(i) - lo; };
-    auto seg_lo = [](int) { return 0; };
-    bool split = false;
-    for (int left = shift; left > 0 && !fix_ties(s, n, full, seg_lo, [n](int) { return n; });) {
-      left = split_ties(s, n, nitems, left, dropped, seg_lo);
-      split = true;
-    }
-    if (split && !whole) {  // the merges go by the kept bits
-      for (int q = threadIdx.x; q < n; q += kRunBlock) s.key[q] = (unsigned)(dropped(s.idx[q]) >> shift);
+    if (shift > 0 && !fix_ties(s, n, full, [](int) { return 0; }, [n](int) { return n; })) {
+      for (int q = threadIdx.x; q < nitems * kRunBlock; q += kRunBlock) {
+        s.key[q] = q < n ? (unsigned)((full(q) - lo) & ((1ull << shift) - 1ull)) : ~0u;
+        s.idx[q] = (unsigned short)q;
+      }
       __syncthreads();
+      radix_bits<Tile>(nitems, shift);
+      for (int q = threadIdx.x; q < nitems * kRunBlock; q += kRunBlock) {
+        const int i = s.idx[q];
+        s.key[q] = i < n ? (unsigned)((full(i) - lo) >> shift) : ~0u;
+      }
+      __syncthreads();
+      radix_bits<Tile>(nitems, width - shift);
     }
   }
   if (whole) {
