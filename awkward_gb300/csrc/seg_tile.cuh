@@ -986,35 +986,35 @@ __device__ __forceinline__ void seg_tile_range(const Op& op,
   if (base >= I1) return;
 
   // From here on lists and elements count from the first of the range, in 32
-  // bits (a range holds fewer than 2^31 of both; the offsets' low words give
-  // the differences).
+  // bits (a range holds fewer than 2^31 of both; the offsets' low words, unsigned,
+  // give the differences).
   using T = store_t<typename Op::In>;
   const T* xr = x + lo;
-  const int* ends = reinterpret_cast<const int*>(offsets + base + 1);
+  const unsigned* ends = reinterpret_cast<const unsigned*>(offsets + base + 1);
   typename Op::Out* to = out + base;
-  const int lists = (int)(I1 - base), first = (int)lo;
+  const int lists = (int)(I1 - base);
+  const unsigned first = (unsigned)lo;
   auto load_end = [&](int l) {
     l = l < lists ? l : lists - 1;
     return __ldg(ends + 2 * (long long)l);  // (nothing waits for it here)
   };
   if constexpr (kDirect<Op>) {
-    const int n = (int)((unsigned)__ldg(ends + 2 * (long long)(lists - 1)) - (unsigned)first);
+    const int n = (int)(__ldg(ends + 2 * (long long)(lists - 1)) - first);
     bool direct = n >= (long long)lists * kWarpList;
     for (int b = 0; b < lists && direct; b += 32) {
-      const int en = load_end(b + lane), up = __shfl_up_sync(kFull, en, 1);
-      const int st = lane ? up : b ? load_end(b - 1) : first;
-      direct = __all_sync(kFull, (unsigned)en - (unsigned)st <= (unsigned)kSpan<T>);
+      const unsigned en = load_end(b + lane), up = __shfl_up_sync(kFull, en, 1);
+      const unsigned st = lane ? up : b ? load_end(b - 1) : first;
+      direct = __all_sync(kFull, en - st <= (unsigned)kSpan<T>);
     }
     if (direct) {
       WalkState<Op> state;
       if constexpr (WalkOf<Op>::value == Walk::kExtremum) state.ident = ident_key(op);
       for (int b = 0; b < lists; b += 32) {
         const int c = lists - b < 32 ? lists - b : 32;
-        const int en = load_end(b + lane), up = __shfl_up_sync(kFull, en, 1);
-        const int st = lane ? up : b ? load_end(b - 1) : first;
-        const int at = (int)((unsigned)st - (unsigned)first);
-        typename Op::Out v = direct_results(op, xr, c, lane < c ? (int)((unsigned)en - (unsigned)st) : 0,
-                                            at, lane, state);
+        const unsigned en = load_end(b + lane), up = __shfl_up_sync(kFull, en, 1);
+        const unsigned st = lane ? up : b ? load_end(b - 1) : first;
+        typename Op::Out v = direct_results(op, xr, c, lane < c ? (int)(en - st) : 0, (int)(st - first),
+                                            lane, state);
         if constexpr (WalkOf<Op>::value == Walk::kArg) v = v < 0 ? v : v + lo;
         if (lane < c) to[b + lane] = v;
       }
@@ -1027,9 +1027,9 @@ __device__ __forceinline__ void seg_tile_range(const Op& op,
   struct Round {
     int nl, rel, n, hi, shift;
   };
-  auto plan = [&](int b, int l, int en, int buf) {
+  auto plan = [&](int b, int l, unsigned en, int buf) {
     Round r;
-    r.rel = en - (first + l);
+    r.rel = (int)(en - (first + (unsigned)l));
     const unsigned m = __ballot_sync(kFull, (unsigned)r.rel > (unsigned)kSpan<T> || lane >= lists - b);
     r.nl = m ? __ffs(m) - 1 : 32;
     r.n = __shfl_sync(kFull, r.rel, r.nl ? r.nl - 1 : 0);
@@ -1048,7 +1048,7 @@ __device__ __forceinline__ void seg_tile_range(const Op& op,
   int at = 0, begin = 0, which = 0;
   Round now = plan(0, 0, load_end(lane), 0);
   int next = now.nl ? now.nl : 1;
-  int en = load_end(next + lane);
+  unsigned en = load_end(next + lane);
   while (true) {
     Round ahead{0, 0, 0, 0, 0};
     if (next < lists) {
