@@ -108,14 +108,20 @@ __global__ void max_backward_kernel(T* __restrict__ gx, const T* __restrict__ go
 // longest list chooses how many lanes share a list, 4 to 32, and how many elements
 // a lane has, 6 at most; these are loaded once, kept in registers, reduced with
 // shuffles among the list's lanes and stored, the loads of several steps in flight.
-// A round with a list of more than kSoftLongest elements goes list by list, a warp
-// on each, in three passes.  Bound by the instructions of places past the lists' ends
-// at first, by HBM from mean 16 on: 1M lists, us (forward, backward with y kept):
-// mean 4 44, 43 -> 21, 21; mean 16 61, 68 -> 36, 46 (128 and 192 MB, 19 and 28 us);
-// 20000 lists of mean 500 188, 425 -> 113, 208.  Before, tiles of 64 lists were
-// staged in shared memory, one thread reducing each list.
+// Lists of more than kSoftLongest elements go one by one, a warp on each, in three
+// passes.  Where the mean is above that, or few lists leave most of the chip idle, a
+// warp has fewer lists, and those of more than kSoftWarp elements are taken by the
+// whole CTA.  (Only there: the barrier that the CTA's lists need cost rounds of short
+// lists 10 to 15 %.)  Bound by the instructions of places past the lists' ends at
+// first, by HBM from mean 16 on: 1M lists, us (forward, backward with y kept): mean 4
+// 44, 43 -> 21, 22; mean 16 61, 68 -> 36, 47 (128 and 192 MB, 19 and 28 us); 20000
+// lists of mean 500 188, 425 -> 42, 68; 32 lists of 100000 20000, 19100 -> 392, 347.
+// Before, tiles of 64 lists were staged in shared memory, one thread reducing each
+// list; 32 lists to every warp, a long one making all 32 go one by one, had taken
+// 45700 and 39200 us for the last.
 constexpr int kSoftThreads = 128;
 constexpr int kSoftLongest = 32 * 6;
+constexpr int kSoftWarp = 1024;  // longest list of a CTA of few lists taken by one warp
 constexpr int kSoftFlight = 24;  // 4-byte words a lane has in flight
 
 template <class T, class F>
@@ -131,6 +137,37 @@ template <class T>
 __device__ __forceinline__ T lanes_sum(T v, int lanes) {
   return lanes_reduce(v, lanes, [](T a, T b) { return a + b; });
 }
+
+// The threads that take one long list between them: a warp, or the CTA.
+struct TeamWarp {
+  static constexpr int kLanes = 32;
+  int lane;
+  template <class T>
+  __device__ __forceinline__ T max(T v) const { return lanes_max(v, 32); }
+  template <class T>
+  __device__ __forceinline__ T sum(T v) const { return lanes_sum(v, 32); }
+};
+struct TeamBlock {
+  static constexpr int kLanes = kSoftThreads;
+  int lane;
+  float* part;  // a place for each warp
+  template <class F>
+  __device__ __forceinline__ float join(float v, F f) const {
+    __syncthreads();  // (the places may still be read)
+    if ((lane & 31) == 0) part[lane >> 5] = v;
+    __syncthreads();
+    v = part[0];
+#pragma unroll
+    for (int w = 1; w < kLanes / 32; w++) v = f(v, part[w]);
+    return v;
+  }
+  __device__ __forceinline__ float max(float v) const {
+    return join(lanes_max(v, 32), [](float a, float b) { return max_t(a, b); });
+  }
+  __device__ __forceinline__ float sum(float v) const {
+    return join(lanes_sum(v, 32), [](float a, float b) { return a + b; });
+  }
+};
 
 // What becomes of a list whose elements a lane group holds: in[0] = x (forward), or
 // in[0] = gy and in[1] = the saved y or x (backward).
@@ -153,15 +190,15 @@ struct SoftForward {
 #pragma unroll
     for (int k = 0; k < N; k++) out[k] *= inv;
   }
-  // one list by a warp: x[0 .. n)
-  template <class T>
-  __device__ __forceinline__ static void list(T* out, const T* const (&in)[1], long long n, int lane) {
+  // one list, x[0 .. n), by a team (TeamWarp or TeamBlock)
+  template <class T, class Team>
+  __device__ __forceinline__ static void list(T* out, const T* const (&in)[1], long long n, Team team) {
     T m = -INFINITY, sum = 0;
-    for (long long q = lane; q < n; q += 32) m = max_t(m, in[0][q]);
-    m = lanes_max(m, 32);
-    for (long long q = lane; q < n; q += 32) sum += out[q] = exp_t(in[0][q] - m);
-    const T inv = T(1) / lanes_sum(sum, 32);
-    for (long long q = lane; q < n; q += 32) out[q] *= inv;
+    for (long long q = team.lane; q < n; q += Team::kLanes) m = max_t(m, in[0][q]);
+    m = team.max(m);
+    for (long long q = team.lane; q < n; q += Team::kLanes) sum += out[q] = exp_t(in[0][q] - m);
+    const T inv = T(1) / team.sum(sum);
+    for (long long q = team.lane; q < n; q += Team::kLanes) out[q] *= inv;
   }
 };
 // d x_j = y_j (g_j - sum_k g_k y_k)
@@ -177,12 +214,12 @@ struct SoftBackwardSaved {
 #pragma unroll
     for (int k = 0; k < N; k++) out[k] = in[1][k] * (in[0][k] - dot);
   }
-  template <class T>
-  __device__ __forceinline__ static void list(T* out, const T* const (&in)[2], long long n, int lane) {
+  template <class T, class Team>
+  __device__ __forceinline__ static void list(T* out, const T* const (&in)[2], long long n, Team team) {
     T dot = 0;
-    for (long long q = lane; q < n; q += 32) dot += in[0][q] * in[1][q];
-    dot = lanes_sum(dot, 32);
-    for (long long q = lane; q < n; q += 32) out[q] = in[1][q] * (in[0][q] - dot);
+    for (long long q = team.lane; q < n; q += Team::kLanes) dot += in[0][q] * in[1][q];
+    dot = team.sum(dot);
+    for (long long q = team.lane; q < n; q += Team::kLanes) out[q] = in[1][q] * (in[0][q] - dot);
   }
 };
 // The same with y computed again from x.
@@ -207,33 +244,33 @@ struct SoftBackward {
 #pragma unroll
     for (int k = 0; k < N; k++) out[k] = out[k] * inv * (in[0][k] - dot);
   }
-  template <class T>
-  __device__ __forceinline__ static void list(T* out, const T* const (&in)[2], long long n, int lane) {
+  template <class T, class Team>
+  __device__ __forceinline__ static void list(T* out, const T* const (&in)[2], long long n, Team team) {
     T m = -INFINITY, sum = 0, gsum = 0;
-    for (long long q = lane; q < n; q += 32) m = max_t(m, in[1][q]);
-    m = lanes_max(m, 32);
-    for (long long q = lane; q < n; q += 32) {
+    for (long long q = team.lane; q < n; q += Team::kLanes) m = max_t(m, in[1][q]);
+    m = team.max(m);
+    for (long long q = team.lane; q < n; q += Team::kLanes) {
       const T e = out[q] = exp_t(in[1][q] - m);
       sum += e;
       gsum += in[0][q] * e;
     }
-    const T inv = T(1) / lanes_sum(sum, 32);
-    const T dot = lanes_sum(gsum, 32) * inv;
-    for (long long q = lane; q < n; q += 32)
+    const T inv = T(1) / team.sum(sum);
+    const T dot = team.sum(gsum) * inv;
+    for (long long q = team.lane; q < n; q += Team::kLanes)
       out[q] = out[q] * inv * (in[0][q] - dot);
   }
 };
 
-// One round whose lists have at most LANES * ITEMS elements: lane l holds list l's
-// first element (relative to the pointers) and length.
-template <int LANES, int ITEMS, class Op, class T>
+// One round of `lists` lists (32 when SHARE is) with at most LANES * ITEMS elements:
+// lane l holds list l's first element (relative to the pointers) and length.
+template <int LANES, int ITEMS, int SHARE, class Op, class T>
 __device__ __forceinline__ void soft_round(Op, T* __restrict__ out, const T* const (&in)[Op::kArrays],
-                                           int first, int len, int lane) {
+                                           int first, int len, int lists, int lane) {
   constexpr int kMost = kSoftFlight / ((int)sizeof(T) / 4 * ITEMS * Op::kArrays);
   constexpr int kSteps = kMost >= 4 ? 4 : kMost >= 2 ? 2 : 1;  // steps in flight
   const int i0 = lane % LANES;
 #pragma unroll 1
-  for (int s0 = 0; s0 < LANES; s0 += kSteps) {
+  for (int s0 = 0; SHARE == 32 ? s0 < LANES : s0 * (32 / LANES) < lists; s0 += kSteps) {
     T v[kSteps][Op::kArrays][ITEMS];
     int at[kSteps], left[kSteps];  // the lane's first element, the elements from there on
 #pragma unroll
@@ -259,49 +296,77 @@ __device__ __forceinline__ void soft_round(Op, T* __restrict__ out, const T* con
   }
 }
 
-template <class Op>
+// A warp takes SHARE lists, or (0) a quarter of the CTA's `lists`.
+template <class Op, int SHARE>
 __global__ void __launch_bounds__(kSoftThreads)
     softmax_kernel(float* __restrict__ out, const float* __restrict__ in0, const float* __restrict__ in1,
                    const int64_t* __restrict__ offsets, long long nlists, long long nvalues,
-                   unsigned rounds_blocks) {
+                   int lists, unsigned rounds_blocks) {
   if (blockIdx.x >= rounds_blocks) {  // the elements no list covers
     zero_outside(out, offsets, nlists, nvalues,
                  (blockIdx.x - rounds_blocks) * (long long)kSoftThreads + threadIdx.x,
                  (long long)(gridDim.x - rounds_blocks) * kSoftThreads);
     return;
   }
-  const int lane = threadIdx.x & 31;
-  const long long l0 = (blockIdx.x * (long long)(kSoftThreads / 32) + (threadIdx.x >> 5)) * 32;
-  if (l0 >= nlists) return;
-  const long long l = l0 + lane;
-  const long long begin = __ldg(offsets + (l < nlists ? l : nlists));
-  const long long end = __ldg(offsets + (l < nlists ? l + 1 : nlists));
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int share = SHARE ? SHARE : (lists + 3) / 4;
+  const long long l0 = blockIdx.x * (long long)lists;
+  const long long l = l0 + warp * share + lane;
+  const long long stop = l0 + lists < nlists ? l0 + lists : nlists;
+  const bool act = lane < share && l < stop;
+  const long long begin = __ldg(offsets + (act ? l : stop));
+  const long long end = __ldg(offsets + (act ? l + 1 : stop));
   const long long base = __shfl_sync(0xffffffffu, begin, 0);
   const long long n = end - begin;
   const float* const in[2] = {in0, in1};
+  int len = (int)n;
   if (__any_sync(0xffffffffu, n < 0 || n > kSoftLongest)) {
-    for (int j = 0; j < 32; j++) {
-      const long long b = __shfl_sync(0xffffffffu, begin, j), m = __shfl_sync(0xffffffffu, n, j);
+    // the long ones by the warp (with SHARE 0 up to kSoftWarp elements); all of them
+    // where the round cannot reach its lists by 32-bit places from its first
+    const int most = __shfl_sync(0xffffffffu, end, 31) - base < 1ll << 30 ? kSoftLongest : 0;
+    for (unsigned m = __ballot_sync(0xffffffffu, n > most && (SHARE || n <= kSoftWarp)); m; m &= m - 1) {
+      const int j = __ffs(m) - 1;
+      const long long b = __shfl_sync(0xffffffffu, begin, j);
       const float* p[Op::kArrays];
 #pragma unroll
       for (int a = 0; a < Op::kArrays; a++) p[a] = in[a] + b;
-      if (m > 0) Op::list(out + b, p, m, lane);
+      Op::list(out + b, p, __shfl_sync(0xffffffffu, n, j), TeamWarp{lane});
     }
-    return;
+    if (n < 0 || n > most) len = 0;
   }
-  const float* p[Op::kArrays];
-#pragma unroll
-  for (int a = 0; a < Op::kArrays; a++) p[a] = in[a] + base;
-  const int first = (int)(begin - base), len = (int)n;
   const int longest = __reduce_max_sync(0xffffffffu, len);
-  float* o = out + base;
-  if (longest <= 8) soft_round<4, 2>(Op(), o, p, first, len, lane);
-  else if (longest <= 16) soft_round<4, 4>(Op(), o, p, first, len, lane);
-  else if (longest <= 24) soft_round<4, 6>(Op(), o, p, first, len, lane);
-  else if (longest <= 32) soft_round<8, 4>(Op(), o, p, first, len, lane);
-  else if (longest <= 48) soft_round<8, 6>(Op(), o, p, first, len, lane);
-  else if (longest <= 96) soft_round<16, 6>(Op(), o, p, first, len, lane);
-  else soft_round<32, 6>(Op(), o, p, first, len, lane);
+  if (longest > 0) {
+    const float* p[Op::kArrays];
+#pragma unroll
+    for (int a = 0; a < Op::kArrays; a++) p[a] = in[a] + base;
+    const int first = (int)(begin - base);
+    float* o = out + base;
+    if (longest <= 8) soft_round<4, 2, SHARE>(Op(), o, p, first, len, share, lane);
+    else if (longest <= 16) soft_round<4, 4, SHARE>(Op(), o, p, first, len, share, lane);
+    else if (longest <= 24) soft_round<4, 6, SHARE>(Op(), o, p, first, len, share, lane);
+    else if (longest <= 32) soft_round<8, 4, SHARE>(Op(), o, p, first, len, share, lane);
+    else if (longest <= 48) soft_round<8, 6, SHARE>(Op(), o, p, first, len, share, lane);
+    else if (longest <= 96) soft_round<16, 6, SHARE>(Op(), o, p, first, len, share, lane);
+    else soft_round<32, 6, SHARE>(Op(), o, p, first, len, share, lane);
+  }
+  if constexpr (SHARE == 0) {  // the CTA's lists of more than kSoftWarp elements
+    __shared__ long long s_long[kSoftThreads];
+    __shared__ int s_longs;
+    __shared__ float s_part[kSoftThreads / 32];
+    if (!__syncthreads_or(n > kSoftWarp)) return;
+    if (threadIdx.x == 0) s_longs = 0;
+    __syncthreads();
+    if (n > kSoftWarp) s_long[atomicAdd(&s_longs, 1)] = l;
+    __syncthreads();
+    const int longs = s_longs;
+    for (int j = 0; j < longs; j++) {
+      const long long b = __ldg(offsets + s_long[j]);
+      const float* p[Op::kArrays];
+#pragma unroll
+      for (int a = 0; a < Op::kArrays; a++) p[a] = in[a] + b;
+      Op::list(out + b, p, __ldg(offsets + s_long[j] + 1) - b, TeamBlock{(int)threadIdx.x, s_part});
+    }
+  }
 }
 
 // Doubles, whose exponentials and sums fill the narrow 64-bit unit, go by tiles of
@@ -465,26 +530,35 @@ __global__ void __launch_bounds__(kSoftThreads)
     const double* p[Op::kArrays];
 #pragma unroll
     for (int a = 0; a < Op::kArrays; a++) p[a] = in[a] + t.base + t.loc[r];
-    Op::list(out + t.base + t.loc[r], p, t.loc[r + 1] - t.loc[r], threadIdx.x & 31);
+    Op::list(out + t.base + t.loc[r], p, t.loc[r + 1] - t.loc[r], TeamWarp{(int)threadIdx.x & 31});
   }
 }
 
 template <class Op, class T>
 cudaError_t softmax(T* out, const T* in0, const T* in1, const int64_t* offsets, long long nlists,
                     long long nvalues, cudaStream_t s) {
-  // doubles: the most lists, 8 to kTileSoft, of which a tile's elements fit with a
-  // quarter to spare (by the mean length)
+  const long long mean = nvalues / nlists;
   int lists = sizeof(T) == 8 ? kTileSoft : kSoftThreads;
-  if (sizeof(T) == 8)
-    while (lists > 8 && nvalues / nlists * lists > kTileElems / 5 * 4) lists /= 2;
+  if (sizeof(T) == 8) {
+    // doubles: the most lists, 8 to kTileSoft, of which a tile's elements fit with a
+    // quarter to spare (by the mean length)
+    while (lists > 8 && mean * lists > kTileElems / 5 * 4) lists /= 2;
+  } else {
+    // floats: a round of 32 lists per warp where they are short, 8 where few or long
+    // ones would leave most of the chip idle, fewer when a CTA would then take more than
+    // 16384 elements.  With 32 and so, us, forward: 1000 lists of mean 500 103 and 33,
+    // 1000 heavy-tailed lists of mean 60 48 and 17, 60000 of mean 250 81 and 52.
+    while (lists > 32 && (nlists / lists < 2 * device_sm_count() || mean > 192)) lists /= 2;
+    while (lists > 1 && mean * lists > kSoftWarp * 16) lists /= 2;
+  }
   const unsigned blocks = (unsigned)((nlists + lists - 1) / lists);
   const unsigned rest = nvalues > 0 ? 2 * device_sm_count() : 0;
   if constexpr (sizeof(T) == 8)
     softmax_tile_kernel<Op><<<blocks + rest, kSoftThreads, 0, s>>>(out, in0, in1, offsets, nlists,
                                                                    nvalues, lists, blocks);
   else
-    softmax_kernel<Op><<<blocks + rest, kSoftThreads, 0, s>>>(out, in0, in1, offsets, nlists,
-                                                              nvalues, blocks);
+    (lists == kSoftThreads ? softmax_kernel<Op, 32> : softmax_kernel<Op, 0>)<<<
+        blocks + rest, kSoftThreads, 0, s>>>(out, in0, in1, offsets, nlists, nvalues, lists, blocks);
   return cudaGetLastError();
 }
 
