@@ -329,8 +329,7 @@ class GB300Backend:
                 with torch.cuda.stream(stream):
                     ctx.err.fill_(-1)
         finally:
-            with ctx.lock:
-                ctx.taken.remove(taken)
+            ctx.taken.remove(taken)
             if ctx.captured:
                 self._contexts.pop((index, raw), None)
         code = word & ((1 << ERROR_BITS) - 1)
