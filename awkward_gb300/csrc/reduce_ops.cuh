@@ -432,8 +432,9 @@ struct ArgExtremumOp<double, MAX> {
 
 // ---------------------------------------------------------------- short runs
 // Element loaders of the short-run reducers: global memory through the
-// read-only path, or a run staged in shared memory (the double reducers below
-// take only these: their lists in global memory go by the tile walk).
+// read-only path, or a run staged in shared memory (the reducers of doubles below
+// take only these, mapped runs of fused.cu: their lists in global memory go by the
+// tile walk).
 struct LdGlobal {
   template <class T>
   __device__ __forceinline__ T operator()(const T* p) const {
@@ -474,10 +475,10 @@ __device__ __forceinline__ bool raw_key_exact(long long k) {
   return k != 0 && k != -1 && k <= 0x7ff0000000000000LL && k >= (long long)0x800fffffffffffffULL;
 }
 
-template <bool MAX, class Ld = LdGlobal>
+template <bool MAX>
 __device__ __forceinline__ typename ExtremumOp<double, MAX>::Acc run_short(
     const ExtremumOp<double, MAX>& op, const double* p, int n, long long j0, long long st,
-    long long li, Ld ld = Ld{}) {
+    long long li, LdShared ld) {
   const long long* q = reinterpret_cast<const long long*>(p);
   long long best = 0;
   int at = -1;
@@ -496,10 +497,10 @@ __device__ __forceinline__ typename ExtremumOp<double, MAX>::Acc run_short(
   return a;
 }
 
-template <bool MAX, class Ld = LdGlobal>
+template <bool MAX>
 __device__ __forceinline__ typename ArgExtremumOp<double, MAX>::Acc run_short(
     const ArgExtremumOp<double, MAX>& op, const double* p, int n, long long j0, long long st,
-    long long li, Ld ld = Ld{}) {
+    long long li, LdShared ld) {
   const long long* q = reinterpret_cast<const long long*>(p);
   long long best = 0;
   int at = -1;
@@ -536,7 +537,7 @@ __device__ __forceinline__ FxAcc run_short(const FixedSumOp<IN>& op, const IN* p
     // pipes; the float64 partial rides in FxAcc::dp and is added to the
     // rounded fixed-point part at the end (IEEE inf/NaN included).  The
     // result stays within n*eps*sum|x| of the exact sum.
-      const long long* q = reinterpret_cast<const long long*>(p);
+    const long long* q = reinterpret_cast<const long long*>(p);
     const int* qh = reinterpret_cast<const int*>(p) + 1;
     double dsum = 0.0;
     int ebmax = 0, ebmin = 0x7ff00000;
