@@ -19,8 +19,10 @@ kernels, for CUDA tensors:
   ``awkward_ListArray_getitem_next_range`` and the carry
   (src/awkward/contents/listarray.py:795-862).
 
-Sizes that depend on data are read back from the device exactly where
-awkward reads them (the carry length, the total of true mask entries).
+awkward's own steps read sizes that depend on data back from the device where
+awkward reads them (the carry length, the total of true mask entries); the
+one-call functions write into a buffer that is large enough and read size and
+error back with one wait at their end (see _WHOLE_SOURCE, _WHOLE_CONTENT).
 Errors follow awkward's protocol and surface as ``ValueError``.
 """
 
@@ -176,6 +178,9 @@ def index_select(offsets, content, index_offsets, index, with_carry=False):
     content and, with `with_carry`, the carry -- the same outputs as
     getitem_jagged_index without writing and re-reading the carry.  Errors
     are jagged_apply's, raised as ValueError."""
+    offsets = _array("offsets", offsets, torch.int64)
+    index_offsets = _array("index_offsets", index_offsets, torch.int64)
+    index, content = _array("index", index, torch.int64), _array("content", content)
     n = offsets.numel() - 1
     k = index.numel()
     call = _Call(offsets.device)

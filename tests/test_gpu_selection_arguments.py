@@ -131,3 +131,23 @@ def test_range_of_wide_items():
     assert nextoffsets.tolist() == [0, 0, 0, 0] and out.numel() == 0 and out.dtype == x.dtype
     with pytest.raises(RuntimeError, match="cudaError 1$"):
         jagged.getitem_inner_range(off, off, x, 1)
+
+
+@pytest.mark.gpu
+def test_index_arguments():
+    import torch
+
+    from awkward_gb300 import jagged
+
+    off = torch.tensor([0, 9, 3, 9, 5, 9], dtype=torch.int64, device="cuda")
+    ioff = torch.tensor([0, 9, 1, 9, 3, 9], dtype=torch.int64, device="cuda")
+    idx = torch.tensor([2, 9, -1, 9, 0, 9], dtype=torch.int64, device="cuda")
+    x = torch.arange(5, dtype=torch.float32, device="cuda")
+    for k, name in enumerate(("offsets", "index_offsets", "index")):
+        args = [off[::2], x, ioff[::2], idx[::2]]
+        at = (0, 2, 3)[k]
+        args[at] = args[at].to(torch.int32)
+        with pytest.raises(TypeError, match=f"^{name} must have dtype torch.int64"):
+            jagged.index_select(*args)
+    to, out, carry = jagged.index_select(off[::2], x, ioff[::2], idx[::2], with_carry=True)
+    assert to.tolist() == [0, 1, 3] and out.tolist() == [2.0, 4.0, 3.0] and carry.tolist() == [2, 4, 3]
