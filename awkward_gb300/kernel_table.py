@@ -92,64 +92,34 @@ class _Invocation:
         self.keepalive = keepalive
 
 
-class _Pending:
-    """Invocations `first`, `first` + 1, ... of a stream."""
-
-    __slots__ = ("first", "calls")
-
-    def __init__(self, first):
-        self.first = first
-        self.calls = []
-
-    def get(self, number):
-        i = number - self.first
-        return self.calls[i] if 0 <= i < len(self.calls) else None
-
-
 class _StreamContext:
     """Error word and pending invocations of one stream, for all threads that use it.
 
-    Invocations are numbered on through every synchronisation, and a number is
-    given out and its kernel launched under the lock.  So whoever takes the
-    pending ones knows that all of them are on the stream, and an error that a
-    later call leaves in the word has a number of its own."""
+    Invocations are numbered on through every synchronisation: calls[i] is number
+    first + i.  A number is given out and its kernel launched under the lock, and a
+    call stays in the list until the word has been read behind it.  So an error of
+    any thread's call finds its name, whoever reads the word."""
 
     def __init__(self, device):
         self.err = torch.full((1,), -1, dtype=torch.int64, device=device)  # NO_ERROR
         self.address = self.err.data_ptr()
         self.lock = threading.Lock()
-        self.pending = _Pending(0)
-        self.taken = []  # by synchronisations that have not read the word yet
+        self.first = 0
+        self.calls = []
         # (the word of a context made during a capture is filled by the graph's replays)
         self.captured = torch.cuda.is_current_stream_capturing()
 
-    def launch(self, f, cargs, call, index, stream, fault=None):
-        """f(*cargs, number, word, stream) as the next invocation, and the error
-        code `fault` in its name; f's result."""
+    def launched(self):
+        """The number after the last one: all before are on the stream."""
         with self.lock:
-            calls = self.pending.calls
-            number = self.pending.first + len(calls)
-            calls.append(call)
-            rc = f(*cargs, number, self.address, stream)
-            if fault is not None and rc == 0:
-                self.record_error(number, fault, torch.cuda.current_stream(index))
-            return rc
+            return self.first + len(self.calls)
 
-    def take(self):
-        """The pending invocations, for a synchronisation that reads the word next."""
-        with self.lock:
-            p = self.pending
-            self.pending = _Pending(p.first + len(p.calls))
-            self.taken.append(p)
-            return p
-
-    def call(self, number):
-        """The invocation of that number, None when it is no longer known."""
-        for p in (*self.taken, self.pending):
-            c = p.get(number)
-            if c is not None:
-                return c
-        return None
+    def over(self, number):
+        """The calls before `number` are over."""
+        done = number - self.first
+        if done > 0:
+            del self.calls[:done]
+            self.first = number
 
     def record_error(self, invocation, code, stream):
         """Lower the error word to invocation*256 + code on `stream` (as atomicMin does)."""
@@ -241,11 +211,18 @@ class GB300Kernel:
             index = torch.cuda.current_device()
         stream = raw_stream(index)
         ctx = self.backend._context(index, stream)
-        if len(ctx.pending.calls) >= MAX_PENDING_INVOCATIONS:
+        if len(ctx.calls) >= MAX_PENDING_INVOCATIONS:
             self.backend.synchronize(torch.cuda.current_stream(index))
             ctx = self.backend._context(index, stream)
         fault = injected_fault(self.name, self.family) if FAULT_ENV in os.environ else None
-        rc = ctx.launch(self._f, cargs, _Invocation(self.family, keep), index, stream, fault)
+        call = _Invocation(self.family, keep)
+        with ctx.lock:
+            calls = ctx.calls
+            number = ctx.first + len(calls)
+            calls.append(call)
+            rc = self._f(*cargs, number, ctx.address, stream)
+            if fault is not None and rc == 0:
+                ctx.record_error(number, fault, torch.cuda.current_stream(index))
         if rc != 0:
             raise RuntimeError(f"{self.name}: CUDA launch failed with cudaError {rc}")
 
@@ -297,8 +274,11 @@ class GB300Backend:
         index = torch.cuda.current_device()
         stream = raw_stream(index)
         name = "awkward_gb300_selftest_lookback_timeout"
-        rc = self._context(index, stream).launch(_abi.ext_cfunc(name), (int(spin_limit),),
-                                                 _Invocation(name, []), index, stream)
+        ctx = self._context(index, stream)
+        with ctx.lock:
+            number = ctx.first + len(ctx.calls)
+            ctx.calls.append(_Invocation(name, []))
+            rc = _abi.ext_cfunc(name)(int(spin_limit), number, ctx.address, stream)
         if rc != 0:
             raise RuntimeError(f"look-back self-test: CUDA launch failed with cudaError {rc}")
 
@@ -312,26 +292,26 @@ class GB300Backend:
         if ctx is None:
             stream.synchronize()
             return
-        taken = ctx.take()
-        try:
-            # reading the word waits for the current stream; without an error the
-            # word is as good as new and the context stays
-            if stream != current:
-                stream.synchronize()
-            if int(ctx.err.item()) & NO_ERROR == NO_ERROR:
-                return
-            with ctx.lock:  # no launch until the word is clear again
+        launched = ctx.launched()
+        # reading the word waits for the current stream; without an error the
+        # word is as good as new and the context stays
+        if stream != current:
+            stream.synchronize()
+        word = int(ctx.err.item()) & NO_ERROR
+        with ctx.lock:
+            if word != NO_ERROR:  # no launch until the word is clear again
                 stream.synchronize()
                 word = int(ctx.err.item()) & NO_ERROR
-                if word == NO_ERROR:
-                    return  # raised by another thread meanwhile
-                inv = ctx.call(word >> ERROR_BITS)
+            if word != NO_ERROR:  # (else another thread has raised it meanwhile)
+                at = (word >> ERROR_BITS) - ctx.first
+                inv = ctx.calls[at] if 0 <= at < len(ctx.calls) else None
                 with torch.cuda.stream(stream):
                     ctx.err.fill_(-1)
-        finally:
-            ctx.taken.remove(taken)
-            if ctx.captured:
-                self._contexts.pop((index, raw), None)
+            ctx.over(launched)
+        if ctx.captured:
+            self._contexts.pop((index, raw), None)
+        if word == NO_ERROR:
+            return
         code = word & ((1 << ERROR_BITS) - 1)
         if inv is None:  # a call that a graph has launched again
             what = TIMEOUT_MESSAGE if code == TIMEOUT_CODE else f"error {code}"
