@@ -90,11 +90,17 @@ def ext_cfunc(name):
     return f
 
 
+_word_arrays = {}  # by length
+
+
 def read_words(stream, *addresses):
     """The int64 device words at `addresses`, read with one wait for `stream`
     (a raw cudaStream_t)."""
     n = len(addresses)
-    src, dst = (ctypes.c_void_p * n)(*addresses), (ctypes.c_int64 * n)()
+    types = _word_arrays.get(n)
+    if types is None:
+        types = _word_arrays[n] = ctypes.c_void_p * n, ctypes.c_int64 * n
+    src, dst = types[0](*addresses), types[1]()
     rc = ext_cfunc("awkward_gb300_read_words")(ctypes.addressof(dst), ctypes.addressof(src), n, stream)
     if rc != 0:
         raise RuntimeError(f"awkward_gb300_read_words: cudaError {rc}")

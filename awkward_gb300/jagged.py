@@ -60,7 +60,10 @@ class _Call:
     def __init__(self, device):
         self.key = (device.index, raw_stream(device.index))
         self.stream = self.key[1]
-        self.words = _LOCAL.__dict__.setdefault("words", {})
+        try:
+            self.words = _LOCAL.words
+        except AttributeError:
+            self.words = _LOCAL.words = {}
         self.err = self.words.pop(self.key, None)
         if self.err is None:
             self.err = torch.full((1,), -1, dtype=torch.int64, device=device)
@@ -93,11 +96,13 @@ class _Call:
 
 def _array(name, t, dtype=None):
     """`t` as the library reads it: a contiguous CUDA tensor, of `dtype` if that is given."""
+    if type(t) is torch.Tensor and t.is_cuda and t.dtype is (dtype or t.dtype) and t.is_contiguous():
+        return t
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise TypeError(f"{name} must be a CUDA tensor")
     if dtype is not None and t.dtype is not dtype:
         raise TypeError(f"{name} must have dtype {dtype}, not {t.dtype}")
-    return t if t.is_contiguous() else t.contiguous()
+    return t.contiguous()
 
 
 def _mask(mask):

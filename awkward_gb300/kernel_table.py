@@ -109,18 +109,6 @@ class _StreamContext:
         # (the word of a context made during a capture is filled by the graph's replays)
         self.captured = torch.cuda.is_current_stream_capturing()
 
-    def launched(self):
-        """The number after the last one: all before are on the stream."""
-        with self.lock:
-            return self.first + len(self.calls)
-
-    def over(self, number):
-        """The calls before `number` are over."""
-        done = number - self.first
-        if done > 0:
-            del self.calls[:done]
-            self.first = number
-
     def record_error(self, invocation, code, stream):
         """Lower the error word to invocation*256 + code on `stream` (as atomicMin does)."""
         word = invocation * (1 << ERROR_BITS) + code
@@ -284,30 +272,38 @@ class GB300Backend:
 
     def synchronize(self, stream=None):
         """Wait for the stream; raise ValueError for the first failed invocation."""
-        current = torch.cuda.current_stream()
         if stream is None:
-            stream = current
-        index, raw = stream.device.index, stream.cuda_stream
+            index = torch.cuda.current_device()
+            raw, current = raw_stream(index), True
+        else:
+            index, raw = stream.device.index, stream.cuda_stream
+            current = stream == torch.cuda.current_stream()
         ctx = self._contexts.get((index, raw))
         if ctx is None:
-            stream.synchronize()
+            (stream or torch.cuda.current_stream()).synchronize()
             return
-        launched = ctx.launched()
+        with ctx.lock:  # (all calls before this number are on the stream)
+            launched = ctx.first + len(ctx.calls)
         # reading the word waits for the current stream; without an error the
         # word is as good as new and the context stays
-        if stream != current:
+        if not current:
             stream.synchronize()
         word = int(ctx.err.item()) & NO_ERROR
+        inv = None
         with ctx.lock:
             if word != NO_ERROR:  # no launch until the word is clear again
+                stream = stream or torch.cuda.current_stream()
                 stream.synchronize()
                 word = int(ctx.err.item()) & NO_ERROR
-            if word != NO_ERROR:  # (else another thread has raised it meanwhile)
-                at = (word >> ERROR_BITS) - ctx.first
-                inv = ctx.calls[at] if 0 <= at < len(ctx.calls) else None
-                with torch.cuda.stream(stream):
-                    ctx.err.fill_(-1)
-            ctx.over(launched)
+                if word != NO_ERROR:  # (else another thread has raised it meanwhile)
+                    at = (word >> ERROR_BITS) - ctx.first
+                    inv = ctx.calls[at] if 0 <= at < len(ctx.calls) else None
+                    with torch.cuda.stream(stream):
+                        ctx.err.fill_(-1)
+            over = launched - ctx.first
+            if over > 0:
+                del ctx.calls[:over]
+                ctx.first = launched
         if ctx.captured:
             self._contexts.pop((index, raw), None)
         if word == NO_ERROR:
