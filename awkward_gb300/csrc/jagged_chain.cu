@@ -380,8 +380,9 @@ GB_EXPORT int awkward_gb300_jagged_mask_select(int64_t* tooffsets, void* toconte
 
 // The same with the mask's length and the number of elements in the lists' span,
 // or a bound for it, at hand: where mask_compact() says so the call goes by the
-// bitmap of the whole mask.  Lists that reach outside the mask, or hold more than
-// nelements, raise code 0 ("index out of range"), and no mask entry outside is read.
+// bitmap of the whole mask.  Lists that reach outside the mask (or, by the bitmap,
+// hold more than nelements) raise code 0 ("index out of range"), and no mask entry
+// outside is read.
 GB_EXPORT int awkward_gb300_jagged_mask_select_within(int64_t* tooffsets, void* tocontent,
                                                       int64_t* tocarry, const uint8_t* mask,
                                                       int64_t masklen, const int64_t* offsets,

@@ -70,16 +70,17 @@ struct MaskSpan {
   int shift;
   long long nbits;  // shift + elements of the lists' span (no more than the tables hold)
 };
-// The span of lists whose mask has `masklen` entries; *inside is false when it
-// reaches past them or holds more than `nelements`.
+// The span of lists whose mask has `masklen` entries; *inside is false when these are
+// known and it reaches past them or holds more than `nelements`.
 __device__ __forceinline__ MaskSpan mask_span(const uint8_t* mask, long long masklen,
                                               const int64_t* offsets, long long nlists,
                                               long long nelements, bool* inside = nullptr) {
   MaskSpan s;
   s.first = __ldg(offsets);
   long long last = __ldg(offsets + nlists);
-  if (inside) *inside = s.first >= 0 && last <= masklen && last - s.first <= nelements;
+  if (inside) *inside = true;
   if (masklen != kAnyLength) {
+    if (inside) *inside = s.first >= 0 && last <= masklen && last - s.first <= nelements;
     s.first = s.first < 0 ? 0 : s.first > masklen ? masklen : s.first;
     last = last > masklen ? masklen : last;
   }

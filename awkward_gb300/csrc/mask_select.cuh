@@ -47,14 +47,15 @@ __device__ __forceinline__ int bitmap_count(const unsigned* bits, int a, int b) 
   return n;
 }
 
-// A list's end inside the mask: an offset below 0 or past its `masklen` entries
-// raises code 0 ("index out of range") and is taken as the nearest inside.
+constexpr long long kAnyLength = 0x7fffffffffffffffLL;  // masklen of a mask of unknown length
+
+// A list's end inside the mask: an offset below 0 or past its `masklen` entries (when
+// they are known) raises code 0 ("index out of range") and is taken as the nearest inside.
 __device__ __forceinline__ long long end_in_mask(long long o, long long masklen, uint64_t* err) {
-  if (o >= 0 && o <= masklen) return o;
+  if ((o >= 0 && o <= masklen) || masklen == kAnyLength) return o;
   raise_error(err, 0, 0);
   return o < 0 ? 0 : masklen;
 }
-constexpr long long kAnyLength = 0x7fffffffffffffffLL;  // masklen of a mask of unknown length
 
 struct MaskSelectSmem {
   TileSmem tile;
