@@ -15,17 +15,20 @@
 //                        last end is joined to the first result of a later lane
 //                        by shuffles.  Every lane has the same work whatever
 //                        the lengths;
-//   longer               the warp on one list after the other (warp_results).
+//   longer               the warp on one list after the other, or on a few at once
+//                        (warp_results).
 // Lane i then holds the result of list i of the round (coalesced stores).  A
-// list longer than kSpan is reduced by the whole warp from global memory.
+// list longer than kSpan is reduced by the whole warp from global memory, and so,
+// four lists at a time, is a range of lists of 96 to kSpan elements of which a round
+// would hold few (direct_results).
 //
 // The walk before had a lane per list reading from global memory: about 16 cache
 // lines a load, and as many steps as the warp's longest list.  Bound now by the
 // ALU (75-80 %), the earlier one by load latency.  10M lists of Poisson(8),
 // float64: max 174 -> 148 us, argmax 177 -> 153, sum 240 -> 223 (and the sum is
 // exact now).  16M elements in lists of mean 35: sum 95 -> 60 us, max 86 -> 42;
-// heavy-tailed lists of mean 60: max 128 -> 55.  The sum of lists of 100 to 290
-// doubles is the exception (62 -> 74 us; max 72 -> 57).  The lines: with the
+// heavy-tailed lists of mean 60: max 128 -> 55.  The sum of lists of 100 to 288
+// doubles is the exception (mean 100 62 -> 70 us, 220 57 -> 65).  The lines: with the
 // lanes up to 24 elements the sum at mean 16 (24M elements) took 91 us, with 16
 // 83; with 8, lists of mean 5 took up to 40 % longer.  Element-parallel at a
 // mean of 100 the sum took 117 us (16M elements), the warp on each list 74.

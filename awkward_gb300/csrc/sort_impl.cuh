@@ -12,7 +12,7 @@
 // stable order (std::stable_sort's; it is also a valid answer when `stable`
 // is false).  Segments by length:
 //   <= 32      a warp takes 32 segments: keys staged in its shared memory, and
-//              every element counts the keys of its segment that precede it;
+//              every lane sorts its segment in registers by a network;
 //   <= 2048    tiles of whole segments (up to 4095 elements) sorted by one CTA
 //              with a radix sort in shared memory, the segment as last digit;
 //   longer     runs of 16384 sorted by one CTA each with the same radix sort,
@@ -40,7 +40,7 @@ using namespace gb;
 namespace {
 
 constexpr int kSortBlock = 256;
-constexpr int kShortMax = 32;                  // longest segment sorted by counting
+constexpr int kShortMax = 32;                  // longest segment sorted by a lane
 constexpr int kMidMax = 2048;                  // ... in a tile of whole segments
 constexpr int kMidWindow = 2048;               // a tile: the segments that start in a window
 constexpr int kMidItems = 16;                  // 256 x 16 = 4096 slots >= kMidWindow - 1 + kMidMax
